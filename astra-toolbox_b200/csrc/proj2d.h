@@ -53,6 +53,15 @@ struct BP2DLaunch {
     BPView2D views[BP2D_MAX_VIEWS];
 };
 
+// 2D projection from line copies (lines2d.cu): a copy of the image's rows
+// and columns (FP) or of the sinogram's rows (BP) as pairs of neighbouring
+// texels inside a zero border.  B2T_ERR_NO_MEMORY when the copy does not fit
+// (its scratch, or 32-bit offsets): the callers then read the data directly.
+b2t_status fp2d_lines(const b2t_geom2d *g, uint32_t det_supersample, const float *vol, size_t vol_pitch, float *sino,
+                      size_t sino_pitch, int32_t mode, cudaStream_t s);
+b2t_status bp2d_lines(const b2t_geom2d *g, int32_t fbp_weight, const float *sino, size_t sino_pitch, float *vol,
+                      size_t vol_pitch, int32_t mode, cudaStream_t s);
+
 b2t_status validate2d(const b2t_geom2d *g, const char *who);
 void par_fp_view(const b2t_view2d &p, const b2t_dims2d &d, float out_scale, ParFPView &o);
 void bp2d_view(int kind, int fbp, const b2t_view2d &p, BPView2D &o);

@@ -27,24 +27,107 @@ __device__ __forceinline__ float lerp_line(const float *__restrict__ p, long lon
     return fmaf(f, b - a, a);
 }
 
+// Reciprocal: the hardware's approximation (one ulp) and one Newton-Raphson
+// step r + r (1 - x r), whose residual is exact to FP32 in a fused
+// multiply-add; within one ulp of 1 / x.
+__device__ __forceinline__ float rcp_approx(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_newton(float x)
+{
+    const float r = rcp_approx(x);
+    return fmaf(r, fmaf(-x, r, 1.0f), r);
+}
+
+// Partial sums of a line integral and of a pixel's backprojection: the slices
+// (views) are cut into this many ranges of equal length, each summed on its
+// own and the partial sums then added in order.  The fixed cut lets the line
+// kernels (lines2d.cu) give the ranges of a short problem to different warps
+// and still return the bits of the kernels that run them one after another.
+constexpr int FP2D_PARTS = 4;
+constexpr int BP2D_PARTS = 8;
+
+__host__ __device__ __forceinline__ int part_begin(int p, int n, int parts)
+{
+    return (int)((long long)n * p / parts);
+}
+
+// A ray: sample position q(slice) = A slice + B in texels (texel i at q = i)
+// of the line along the other axis; horizontal: slices are columns.
+struct Ray2D {
+    float A, B, corr;
+    bool horizontal;
+};
+
+// Sub-ray r of R of detector det of a parallel view (corr: see V.corr).
+__device__ __forceinline__ Ray2D par_ray2d(const ParFPView &V, int det, int r, int R)
+{
+    Ray2D q;
+    q.A = V.slicestep;
+    q.B = fmaf((float)det + (0.5f + (float)r) / (float)R - 0.5f, V.detstep, V.p0) - 0.5f;
+    q.corr = V.corr;
+    q.horizontal = !V.vertical;
+    return q;
+}
+
+// Sub-ray r of R of detector det of a fan view, scaled for the mean over R.
+__device__ __forceinline__ Ray2D fan_ray2d(const b2t_view2d &V, int W, int H, int det, int r, int R, float out_scale)
+{
+    Ray2D q;
+    // per-ray orientation choice, in float as the reference evaluates it
+    const float fdx = fabsf(fmaf((float)det, V.det_u[0], V.det_s[0]) + 0.5f - V.src[0]);
+    const float fdy = fabsf(fmaf((float)det, V.det_u[1], V.det_s[1]) + 0.5f - V.src[1]);
+    q.horizontal = !(fdy > fdx);
+    // ray set-up in FP64: the source sits far from the origin
+    const double fdet = det + (0.5 + r) / (double)R;
+    const double DX = V.det_s[0] + fdet * V.det_u[0];
+    const double DY = V.det_s[1] + fdet * V.det_u[1];
+    if (q.horizontal) {
+        const double alpha = (V.src[1] - DY) / (V.src[0] - DX);
+        const double beta = V.src[1] - alpha * V.src[0];
+        q.corr = (float)(sqrt(alpha * alpha + 1.0) * out_scale / R);
+        q.B = (float)(-alpha * (0.5 - 0.5 * W) - beta + 0.5 * H - 0.5);
+        q.A = (float)-alpha;
+    } else {
+        const double alpha = (V.src[0] - DX) / (V.src[1] - DY);
+        const double beta = V.src[0] - alpha * V.src[1];
+        q.corr = (float)(sqrt(alpha * alpha + 1.0) * out_scale / R);
+        q.B = (float)(-alpha * (0.5 - 0.5 * H) + beta + 0.5 * W - 0.5);
+        q.A = (float)-alpha;
+    }
+    return q;
+}
+
+// Sum of the samples of a ray over slices s0, s0 + ds, ...; with ds = 1 from
+// slice 0 all of them, in FP2D_PARTS partial sums.
+__device__ __forceinline__ float sum_ray2d(const float *vol, long long pitch, int W, int H, const Ray2D &q, int s0,
+                                           int ds)
+{
+    const int n0 = q.horizontal ? W : H, n = q.horizontal ? H : W;
+    const long long st0 = q.horizontal ? 1 : pitch, st = q.horizontal ? pitch : 1;
+    float tot = 0.0f;
+    const int parts = ds == 1 ? FP2D_PARTS : 1;
+    for (int p = 0; p < parts; ++p) {
+        const int end = part_begin(p + 1, n0, parts);
+        float sum = 0.0f;
+        for (int sl = part_begin(p, n0, parts) + s0; sl < end; sl += ds)
+            sum += lerp_line(vol + sl * st0, st, n, fmaf((float)sl, q.A, q.B));
+        tot += sum;
+    }
+    return tot;
+}
+
 // Parallel-beam line integral of detector `det` (R sub-rays), scaled; over
 // slices s0, s0 + ds, ... (all slices by default; a partial sum otherwise).
 __device__ __forceinline__ float fp2d_par_ray(const float *vol, long long pitch, int W, int H, const ParFPView &V,
                                               int det, int R, int s0 = 0, int ds = 1)
 {
     float acc = 0.0f;
-    for (int r = 0; r < R; ++r) {
-        const float p0 = fmaf((float)det + (0.5f + (float)r) / (float)R - 0.5f, V.detstep, V.p0);
-        if (!V.vertical) {
-            // slices are columns; the sample moves along the rows
-            for (int sl = s0; sl < W; sl += ds)
-                acc += lerp_line(vol + sl, pitch, H, fmaf((float)sl, V.slicestep, p0) - 0.5f);
-        } else {
-            for (int sl = s0; sl < H; sl += ds)
-                acc += lerp_line(vol + (long long)sl * pitch, 1, W, fmaf((float)sl, V.slicestep, p0) - 0.5f);
-        }
-    }
-    return acc * (V.corr / (float)R);
+    for (int r = 0; r < R; ++r) acc += sum_ray2d(vol, pitch, W, H, par_ray2d(V, det, r, R), s0, ds);
+    return __fmul_rn(acc, V.corr / (float)R);  // (not fused into an accumulating caller)
 }
 
 // Fan-beam line integral of detector `det` (R sub-rays), scaled; over slices
@@ -52,74 +135,56 @@ __device__ __forceinline__ float fp2d_par_ray(const float *vol, long long pitch,
 __device__ __forceinline__ float fp2d_fan_ray(const float *vol, long long pitch, int W, int H, const b2t_view2d &V,
                                               int det, int R, float out_scale, int s0 = 0, int ds = 1)
 {
-    // per-ray orientation choice, in float as the reference evaluates it
-    const float fdx = fabsf(fmaf((float)det, V.det_u[0], V.det_s[0]) + 0.5f - V.src[0]);
-    const float fdy = fabsf(fmaf((float)det, V.det_u[1], V.det_s[1]) + 0.5f - V.src[1]);
-    const bool horizontal = !(fdy > fdx);
     float acc = 0.0f;
     for (int r = 0; r < R; ++r) {
-        // ray set-up in FP64: the source sits far from the origin
-        const double fdet = det + (0.5 + r) / (double)R;
-        const double DX = V.det_s[0] + fdet * V.det_u[0];
-        const double DY = V.det_s[1] + fdet * V.det_u[1];
-        float sum = 0.0f, corr;
-        if (horizontal) {
-            const double alpha = (V.src[1] - DY) / (V.src[0] - DX);
-            const double beta = V.src[1] - alpha * V.src[0];
-            corr = (float)(sqrt(alpha * alpha + 1.0) * out_scale / R);
-            const float y0 = (float)(-alpha * (0.5 - 0.5 * W) - beta + 0.5 * H - 0.5);
-            const float dy = (float)-alpha;
-            for (int sl = s0; sl < W; sl += ds) sum += lerp_line(vol + sl, pitch, H, fmaf((float)sl, dy, y0));
-        } else {
-            const double alpha = (V.src[0] - DX) / (V.src[1] - DY);
-            const double beta = V.src[0] - alpha * V.src[1];
-            corr = (float)(sqrt(alpha * alpha + 1.0) * out_scale / R);
-            const float x0 = (float)(-alpha * (0.5 - 0.5 * H) + beta + 0.5 * W - 0.5);
-            const float dx = (float)-alpha;
-            for (int sl = s0; sl < H; sl += ds)
-                sum += lerp_line(vol + (long long)sl * pitch, 1, W, fmaf((float)sl, dx, x0));
-        }
-        acc = fmaf(sum, corr, acc);
+        const Ray2D q = fan_ray2d(V, W, H, det, r, R, out_scale);
+        acc = fmaf(sum_ray2d(vol, pitch, W, H, q, s0, ds), q.corr, acc);
     }
     return acc;
 }
 
 // Backprojection sum of pixel (X, Y) over views [0, nviews) of `views`
-// (sinogram rows row0 .. row0 + nviews - 1), R x R sub-pixels, unscaled.
+// (sinogram rows row0 .. row0 + nviews - 1), R x R sub-pixels, unscaled, in
+// BP2D_PARTS partial sums.
 __device__ __forceinline__ float bp2d_pixel(const float *sino, long long sino_pitch, int row0, int nviews,
                                             const BPView2D *views, int W, int H, int ndet, int R, int kind, int fbp,
                                             int X, int Y)
 {
     const float sub = 1.0f / (float)R;
-    float acc = 0.0f;
-    for (int i = 0; i < nviews; ++i) {
-        const BPView2D &C = views[i];
-        const float *row = sino + (long long)(row0 + i) * sino_pitch;
-        for (int ix = 0; ix < R; ++ix) {
-            for (int iy = 0; iy < R; ++iy) {
-                float x = (float)X - 0.5f * (float)W + 0.5f;
-                float y = (float)Y - 0.5f * (float)H + 0.5f;
-                if (R > 1) {
-                    x += -0.5f + 0.5f * sub + (float)ix * sub;
-                    y += -0.5f + 0.5f * sub + (float)iy * sub;
-                }
-                if (kind == B2T_GEOM_PAR2D) {
-                    // T = x c - y s + offset (par_bp.cu:78-81)
-                    const float T = fmaf(x, C.c[0], fmaf(-y, C.c[1], C.c[2]));
-                    acc = fmaf(lerp_line(row, 1, ndet, T - 0.5f), C.c[3], acc);
-                } else {
-                    // world y is flipped (fan_bp.cu:73)
-                    const float yw = -y;
-                    const float num = fmaf(x, C.c[1], fmaf(yw, C.c[2], C.c[0]));
-                    const float den = fmaf(x, C.c[4], fmaf(yw, C.c[5], C.c[3]));
-                    const float fr = 1.0f / den;
-                    const float w = fbp ? fr * fr : fr;
-                    acc = fmaf(lerp_line(row, 1, ndet, num * fr - 0.5f), w, acc);
+    float tot = 0.0f;
+    for (int p = 0; p < BP2D_PARTS; ++p) {
+        const int end = part_begin(p + 1, nviews, BP2D_PARTS);
+        float acc = 0.0f;
+        for (int i = part_begin(p, nviews, BP2D_PARTS); i < end; ++i) {
+            const BPView2D &C = views[i];
+            const float *row = sino + (long long)(row0 + i) * sino_pitch;
+            for (int ix = 0; ix < R; ++ix) {
+                for (int iy = 0; iy < R; ++iy) {
+                    float x = (float)X - 0.5f * (float)W + 0.5f;
+                    float y = (float)Y - 0.5f * (float)H + 0.5f;
+                    if (R > 1) {
+                        x += -0.5f + 0.5f * sub + (float)ix * sub;
+                        y += -0.5f + 0.5f * sub + (float)iy * sub;
+                    }
+                    if (kind == B2T_GEOM_PAR2D) {
+                        // T - 1/2, T = x c - y s + offset (par_bp.cu:78-81)
+                        const float q = fmaf(x, C.c[0], fmaf(-y, C.c[1], C.c[2] - 0.5f));
+                        acc = fmaf(lerp_line(row, 1, ndet, q), C.c[3], acc);
+                    } else {
+                        // world y is flipped (fan_bp.cu:73)
+                        const float yw = -y;
+                        const float num = fmaf(x, C.c[1], fmaf(yw, C.c[2], C.c[0]));
+                        const float den = fmaf(x, C.c[4], fmaf(yw, C.c[5], C.c[3]));
+                        const float fr = rcp_newton(den);
+                        const float w = fbp ? fr * fr : fr;
+                        acc = fmaf(lerp_line(row, 1, ndet, fmaf(num, fr, -0.5f)), w, acc);
+                    }
                 }
             }
         }
+        tot += acc;
     }
-    return acc;
+    return tot;
 }
 
 }  // namespace b2t
