@@ -141,6 +141,14 @@ template <typename T> __device__ __forceinline__ elem_t<T, true> splat2(float x)
     else return x;
 }
 
+// Reciprocal to one unit in the last place.
+__device__ __forceinline__ float rcp_approx(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // Bilinear sample with weights fu (along u) and fv (along v) from element p
 // of shared memory (GLOBAL false) or of the padded projections in global
 // memory, rows rs elements apart.
@@ -206,13 +214,14 @@ template <bool CIRC> __device__ __forceinline__ BPView view_rec(const BPTmaLaunc
 
 // Per-view record written by the producer warp: the tile's origin in padded
 // texels (u0, v0), its first ring row and its row count (0: the footprint does
-// not fit a tile, read global memory), and for circular geometries the
-// view's coefficients folded into affine forms of the thread's offset
-// (lx, ly) inside the CTA's block at the block's first z slice, with the
-// tile origin absorbed:
-//   cone:     U = (cu.w + cu.x lx + cu.y ly) / D,  V_j = (cv.w + cv.x lx + cv.y ly + j cv.z) / D,
-//             D = cd.w + cd.x lx + cd.y ly
+// not fit a tile, read global memory), and the view's coefficients folded
+// into affine forms of the thread's offset (lx, ly) inside the CTA's block and
+// of the voxel's offset j from the block's first z slice, with the tile
+// origin absorbed:
+//   cone:     U_j = (cu.w + cu.x lx + cu.y ly + j cu.z) / D_j,  V_j = (cv.w + cv.x lx + cv.y ly + j cv.z) / D_j,
+//             D_j = cd.w + cd.x lx + cd.y ly + j cd.z
 //   parallel: the same without the division; cd.w is the ray weight
+// (circular geometries: cu.z = cd.z = 0, U and D are the column's).
 // U and V are tile-relative sample positions (texel k = floor, weight frac on
 // k + 1).
 struct StageInfo {
@@ -309,17 +318,17 @@ __device__ __noinline__ void bp_produce(const BPTmaLaunch &L, E *ring, uint64_t 
                     r.nrows = rows;
                 }
             }
-            if (CIRC && r.nrows > 0) {
+            if (r.nrows > 0) {
                 // sample position in tile texels: c + 1.5 - origin (c the
                 // continuous detector coordinate, origin the padded index)
                 const double ox = bx0, oy = by0, oz = bz0;
                 if (KIND == B2T_GEOM_CONE) {
-                    r.cu = fold_form(W.nu, W.den, 1.5 - r.u0, ox, oy, oz, false);
+                    r.cu = fold_form(W.nu, W.den, 1.5 - r.u0, ox, oy, oz, !CIRC);
                     r.cv = fold_form(W.nv, W.den, 1.5 - r.v0, ox, oy, oz, true);
-                    r.cd = fold_form(W.den, W.den, 0.0, ox, oy, oz, false);
+                    r.cd = fold_form(W.den, W.den, 0.0, ox, oy, oz, !CIRC);
                 } else {
                     const float4 one = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-                    r.cu = fold_form(W.nu, one, 1.5 - r.u0, ox, oy, oz, false);
+                    r.cu = fold_form(W.nu, one, 1.5 - r.u0, ox, oy, oz, !CIRC);
                     r.cv = fold_form(W.nv, one, 1.5 - r.v0, ox, oy, oz, true);
                     r.cd = make_float4(0.0f, 0.0f, 0.0f, W.den.w);
                 }
@@ -552,7 +561,90 @@ __global__ void __launch_bounds__(288, BPT_CTAS_PER_SM) bp3d_tma_kernel(const __
                 done = true;
             }
         }
-        if (done) ++n_fast;
+        if (!CIRC && active && hd.w > 0) {
+            // any orientation: u, v and the weight of every voxel, from the
+            // folded forms (tile-relative positions: a few dozen texels, so
+            // one-ulp reciprocals leave smaller errors than full-range
+            // detector coordinates would)
+            const float4 cu = info[slot].cu, cv = info[slot].cv, cd = info[slot].cd;
+            const float au = fmaf(ly, cu.y, fmaf(lx, cu.x, cu.w)), av = fmaf(ly, cv.y, fmaf(lx, cv.x, cv.w));
+            const float ad = KIND == B2T_GEOM_CONE ? fmaf(ly, cd.y, fmaf(lx, cd.x, cd.w)) : 1.0f;
+            const float M = 12582912.0f;
+            // U_j and V_j are monotone in j while D stays positive, so the
+            // column is inside the tile when its ends are, a texel from the
+            // edges for the rounding between them
+            const float jl = (float)(ZB - 1);
+            float ul = fmaf(jl, cu.z, au), vl = fmaf(jl, cv.z, av), uf = au, vf = av;
+            bool in = true;
+            if (KIND == B2T_GEOM_CONE) {
+                const float dl = fmaf(jl, cd.z, ad);
+                in = ad > 0.0f && dl > 0.0f;
+                const float f0 = rcp_approx(ad), f1 = rcp_approx(dl);
+                uf *= f0;
+                vf *= f0;
+                ul *= f1;
+                vl *= f1;
+            }
+            in = in && fminf(uf, ul) >= 1.0f && fmaxf(uf, ul) < (float)(BU - 2) && fminf(vf, vl) >= 1.0f &&
+                 fmaxf(vf, vl) < (float)(hd.w - 2);
+            if (in) {
+                constexpr uint32_t ROWB = BU * sizeof(E);
+                const uint32_t rowb = L.tile_row_bytes;  // (a register, as above)
+                const uint32_t abase = smem_u32(tile) - 0x4B400000u * rowb - 0x4B400000u * (uint32_t)sizeof(E);
+                const uint64_t au2 = pk2(au, au), av2 = pk2(av, av), ad2 = pk2(ad, ad);
+                const uint64_t zu2 = pk2(cu.z, cu.z), zv2 = pk2(cv.z, cv.z), zd2 = pk2(cd.z, cd.z);
+                const uint64_t M2 = pk2(M, M), nM2 = pk2(-M, -M), two2 = pk2(2.0f, 2.0f);
+                uint64_t j2 = pk2(0.0f, 1.0f);
+                using H2 = elem_t<T, true>;
+#pragma unroll
+                for (int j = 0; j < ZB; j += 2, j2 = add2(j2, two2)) {
+                    uint64_t qu = fma2(j2, zu2, au2), qv = fma2(j2, zv2, av2), w2;
+                    if constexpr (KIND == B2T_GEOM_CONE) {
+                        const float2 d = upk2(fma2(j2, zd2, ad2));
+                        const uint64_t fr = pk2(rcp_approx(d.x), rcp_approx(d.y));
+                        qu = mul2(qu, fr);
+                        qv = mul2(qv, fr);
+                        w2 = KER == B2T_KER_2D_WEIGHTING ? fr : mul2(fr, fr);
+                    } else {
+                        w2 = pk2(cd.w, cd.w);
+                    }
+                    const uint64_t tu = add2_rd(qu, M2), tv = add2_rd(qv, M2);
+                    const uint64_t fu2 = sub2(qu, add2(tu, nM2)), fv2 = sub2(qv, add2(tv, nM2));
+                    const float2 ku = upk2(tu), kv = upk2(tv);
+                    const uint32_t a0 = (uint32_t)__float_as_int(kv.x) * rowb +
+                                        ((uint32_t)__float_as_int(ku.x) * (uint32_t)sizeof(E) + abase);
+                    const uint32_t a1 = (uint32_t)__float_as_int(kv.y) * rowb +
+                                        ((uint32_t)__float_as_int(ku.y) * (uint32_t)sizeof(E) + abase);
+                    uint64_t ra, rb;
+                    if constexpr (PAIR) {
+                        const float2 fus = upk2(fu2);
+                        float2 ab[2];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const uint32_t c0 = lds_b32<0>(h ? a1 : a0), c1 = lds_b32<4>(h ? a1 : a0);
+                            const float2 x0 = pair_f2<T>(*reinterpret_cast<const H2 *>(&c0));
+                            const float2 x1 = pair_f2<T>(*reinterpret_cast<const H2 *>(&c1));
+                            const float f = h ? fus.y : fus.x;
+                            ab[h] = make_float2(fmaf(f, x1.x - x0.x, x0.x), fmaf(f, x1.y - x0.y, x0.y));
+                        }
+                        ra = pk2(ab[0].x, ab[1].x);
+                        rb = pk2(ab[0].y, ab[1].y);
+                    } else {
+                        const uint64_t v00 = pk2(lds_sh<T, 0>(a0), lds_sh<T, 0>(a1));
+                        const uint64_t v10 = pk2(lds_sh<T, 4>(a0), lds_sh<T, 4>(a1));
+                        const uint64_t v01 = pk2(lds_sh<T, (int)ROWB>(a0), lds_sh<T, (int)ROWB>(a1));
+                        const uint64_t v11 = pk2(lds_sh<T, (int)ROWB + 4>(a0), lds_sh<T, (int)ROWB + 4>(a1));
+                        ra = fma2(fu2, sub2(v10, v00), v00);
+                        rb = fma2(fu2, sub2(v11, v01), v01);
+                    }
+                    const float2 r = upk2(fma2(fma2(fv2, sub2(rb, ra), ra), w2, pk2(acc[j], acc[j + 1])));
+                    acc[j] = r.x;
+                    acc[j + 1] = r.y;
+                }
+                done = true;
+            }
+        }
+        if (CIRC && done) ++n_fast;
         else if (active) ++n_general;
         else ++n_idle;
         if (active && !done) {
