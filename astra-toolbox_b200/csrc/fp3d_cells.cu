@@ -565,7 +565,7 @@ b2t_status build_cells_t(const b2t_geom3d *g, const void *vol, size_t vol_pitch,
             // slab copy for the TMA-staged kernel (fp3d_slab.cu)
             if (!c.mem[dir]) c.mem[dir].reset(new Scratch);
             B2T_TRY(c.mem[dir]->alloc(fp_slab_copy_bytes(d, dir), s, "b2t_fp3d scratch (slab copy)"));
-            B2T_TRY(fp_slab_build(d, static_cast<const float *>(vol), vol_pitch, dir, c.mem[dir]->as<void>(), s));
+            B2T_TRY(fp_slab_build(d, vol, vol_pitch, CellDtype<T>::value, dir, c.mem[dir]->as<void>(), s));
             c.slab[dir] = true;
             c.base[dir] = c.mem[dir]->as<void>();
             continue;
@@ -618,12 +618,12 @@ b2t_status project_cells_t(const b2t_geom3d *g, const b2t_params3d *p, const FPC
     for (int dir = 0; dir < 3 && st == B2T_OK; ++dir) {
         if (!need[dir]) continue;
         if (c.slab[dir]) {
-            if (!fp_slab_eligible(g, p, c.dtype, dir, dirs)) {
+            if (!fp_slab_eligible(g, p, dir, dirs)) {
                 st = fail(B2T_ERR_UNSUPPORTED, "b2t_fp3d: views or parameters differ from those the slab copy was "
                                                "built for");
                 break;
             }
-            st = fp_slab_project(g, p, c.base[dir], dir, proj, proj_pitch, mode, dirs, s);
+            st = fp_slab_project(g, p, c.base[dir], dir, proj, proj_pitch, c.dtype, mode, dirs, s);
             continue;
         }
         P.proj = proj;
@@ -727,7 +727,7 @@ b2t_status fp3d_cells_build(const b2t_geom3d *g, const b2t_params3d *p, const vo
     std::vector<int> dirs(g->dims.angles);
     for (uint32_t a = 0; a < g->dims.angles; ++a) dirs[a] = dominant_axis(g->kind, g->views[a], g->dims);
     bool slab[3] = {false, false, false};
-    for (int dir = 0; dir < 2; ++dir) slab[dir] = need[dir] && fp_slab_eligible(g, p, dtype, dir, dirs);
+    for (int dir = 0; dir < 2; ++dir) slab[dir] = need[dir] && fp_slab_eligible(g, p, dir, dirs);
     if (dtype == B2T_F32) return build_cells_t<float>(g, vol, vol_pitch, need, slab, s, c);
     if (dtype == B2T_F16) return build_cells_t<__half>(g, vol, vol_pitch, need, slab, s, c);
     return build_cells_t<__nv_bfloat16>(g, vol, vol_pitch, need, slab, s, c);

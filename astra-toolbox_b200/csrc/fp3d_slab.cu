@@ -14,24 +14,27 @@
 //
 //   - the volume is copied once per call and marching axis into a slab copy
 //     of z-pairs [slice][in-plane texel + 2][z texel + 2] holding
-//     (v[z], v[z + 1] - v[z]) (z contiguous, a zero border of two texels), so
+//     (v[z], v[z + 1] - v[z]) in FP32 (z contiguous, a zero border of two texels), so
 //     a bilinear sample is two 8-byte loads and two FMAs along z;
 //   - a CTA traces SLAB_W consecutive views x SLAB_U consecutive detector
-//     columns x SLAB_ROWS detector rows; a compute warp owns one column, each
-//     lane SLAB_R rows of it (v, v + 32, ...) in both views, so the in-plane
+//     columns x up to SLAB_ROWS detector rows (blocks of equal height); a
+//     compute warp owns one column, each lane SLAB_R rows of it (v, v + 32, ...) in both views, so the in-plane
 //     position, texel split and buffer row of a slice are computed once per
 //     view for SLAB_R rays and the slice's wait and release once for all
 //     SLAB_W x SLAB_R of them;
 //   - a producer warp works out the buffer box of 32 slices at a time (one
 //     slice per lane) from the tile's corner rays (the rays of a detector
 //     rectangle cross a slice in the convex hull of its corners' crossings),
-//     clamped to the zero border, and loads each slice's box with 4-row
-//     cp.async.bulk.tensor boxes of one of two widths (96 or 160 texels;
-//     plain tile loads, no multicast) into one of SLAB_STAGES slice buffers;
+//     clamped to the zero border where it would not fit a buffer otherwise,
+//     and loads each slice's box with 4-row
+//     cp.async.bulk.tensor boxes of one of two widths (128 or 176 texels;
+//     plain tile loads, no multicast) into one of SLAB_SLOTS slice buffers, two
+//     slices a stage;
 //     a box lands densely, so its width is the buffer's row pitch;
 //   - compute warps interpolate from shared memory in FP32.  Samples outside
-//     the volume read the zero border (positions clamped to it on the slices
-//     where some ray of the warp leaves the volume);
+//     the volume read zeros: the load fills the part of a box outside the
+//     slab copy with them, or, where only a clamped box fits a buffer, the
+//     texels are clamped to the zero border;
 //   - a slice whose box does not fit a buffer (extreme magnification) is read
 //     from the slab copy in global memory instead.
 //
@@ -48,6 +51,7 @@
 #include <atomic>
 #include <cstdlib>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "b2t_internal.h"
@@ -71,21 +75,33 @@ namespace {
 constexpr int SLAB_W = 2;                   // views per CTA (every warp traces both)
 constexpr int SLAB_U = 11;                  // detector columns per CTA, one compute warp each
 constexpr int SLAB_R = 5;                   // rows per lane and view: v, v + 32, ... (384 threads:
-                                            // 80 registers at two CTAs per SM, no spills)
+                                            // 80 registers at two CTAs per SM)
 constexpr int SLAB_ROWS = 32 * SLAB_R;      // detector rows per CTA
 constexpr int SLAB_WARPS = SLAB_U;          // compute warps; one more produces
 constexpr int SLAB_THREADS = 32 * (SLAB_WARPS + 1);
-constexpr int SLAB_BY = 24;                 // buffer rows (in-plane texels) per slice
-constexpr int SLAB_WA = 96, SLAB_WB = 160;  // box widths (z-pairs): the buffer row pitch of a slice
-constexpr int SLAB_BOX_Y = 4;               // rows per TMA box
-constexpr int SLAB_STAGES = 3;              // slices in flight
-constexpr int SLAB_SLOT = SLAB_BY * SLAB_WB;  // z-pairs per slice buffer
+// Slice buffers: four of 3584 z-pairs (28 KB) in the 113 KB that two CTAs per
+// SM leave each, as two stages of two slices.  One wait and one release per two
+// slices take about twelve instructions a slice off the warps (of about 150);
+// measured at 512^3 x 720 / 256^3 x 360 (832^2 / 416^2 detectors): three
+// stages of one slice (24 x 160 pairs) 116.9 / 8.84 ms, four stages of one
+// slice 110.2 / 8.52, two stages of two 105.4 / 7.79 and with box widths 128
+// and 176 (wide boxes of rows far from the source fit: 0.7 % of the slices
+// read global memory instead of 2.9 %) 104.8 / 7.76; widths up to 160 109.9 /
+// 7.95, up to 192 (16 rows) 117.3 / 8.16.
+constexpr int SLAB_WA = 128, SLAB_WB = 176;  // box widths (z-pairs): the buffer row pitch of a slice
+constexpr int SLAB_BOX_Y = 4;                // rows per TMA box
+constexpr int SLAB_PER = 2;                  // slices per stage
+constexpr int SLAB_STAGES = 2;               // stages in flight
+constexpr int SLAB_SLOTS = SLAB_PER * SLAB_STAGES;
+constexpr int SLAB_SLOT = 3584;              // z-pairs per slice buffer: boxes of up to SLOT / width rows
 constexpr int SLAB_MAX_VIEWS = 448;
 constexpr long long SLAB_WAIT = 2000000000LL;  // cycles (about a second)
 constexpr float SPLIT_M = 12582912.0f;      // 1.5 * 2^23
 constexpr int SPLIT_BITS = 0x4B400000;      // bits of SPLIT_M
 
-static_assert(SLAB_BY % SLAB_BOX_Y == 0, "buffer made of whole boxes");
+static_assert((SLAB_SLOT * 8) % 128 == 0 && (SLAB_BOX_Y * SLAB_WA * 8) % 128 == 0 && (SLAB_BOX_Y * SLAB_WB * 8) % 128 == 0,
+              "TMA boxes start on 128-byte boundaries");
+static_assert(32 % SLAB_PER == 0, "a producer batch is made of whole stages");
 static_assert(4 * SLAB_W <= 32, "the producer projects the corner rays one per lane");
 
 // The launch record of the FP and of its transpose (bp3d_slab_matched_kernel,
@@ -101,12 +117,14 @@ struct alignas(64) SlabLaunch {
     long long proj_pitch;
     int n0, n1, n2, nu, nv, na;
     int accumulate;
+    int rows;              // detector rows per CTA (a multiple of 32, at most SLAB_ROWS)
     float f1, f2, mul;     // ray length factors and output scale
     int nviews;
     FPView views[SLAB_MAX_VIEWS];
 };
 
-// A slice's buffer: sel 0 / 1 the box width WA / WB, -1 read global memory;
+// A slice's buffer: sel 0 / 1 the box width WA / WB, 2 / 3 the same clamped to
+// the zero border, -1 read global memory;
 // rbase folds the box origin and the texel split's offset into the byte
 // address: texel (k1, k2) at slot + rbase + bits1 * 8 pitch + bits2 * 8
 struct SlabInfo {
@@ -206,7 +224,7 @@ __device__ __forceinline__ void slab_corners(const SlabLaunch &L, int lane, Corn
     const int w = c >> 2, uc = c & 1, vc = (c >> 1) & 1;
     const int vi = min((int)blockIdx.x * SLAB_W + w, L.nviews - 1);
     const int u = (int)blockIdx.y * SLAB_U + (uc ? SLAB_U - 1 : 0);
-    const int v = (int)blockIdx.z * SLAB_ROWS + (vc ? SLAB_ROWS - 1 : 0);
+    const int v = (int)blockIdx.z * L.rows + (vc ? L.rows - 1 : 0);
     float A1, B1h, A2, B2h;
     const float den = ray_setup(L.views[vi], det_uu(L, u), det_vv(L, v), A1, B1h, A2, B2h);
     C.hull = __all_sync(0xffffffffu, den > 1e-6f) || __all_sync(0xffffffffu, den < -1e-6f);
@@ -219,28 +237,42 @@ __device__ __forceinline__ void slab_corners(const SlabLaunch &L, int lane, Corn
     }
 }
 
-// The box of slice sf from the corners' texels, clamped to the zero border,
-// one texel of margin for rounding: in-plane texels [y0, y1], z texels
-// [zlo, z1].  sane: no corner position so large that its texel saturates.
+// The box of slice sf from the corners' texels, one texel of margin for
+// rounding: in-plane texels [y0, y1], z texels [zlo, z1].  CLAMP: clamped to
+// the zero border, for samples whose texels are clamped to it; else the
+// texels as they are, which outside the volume a TMA load fills with zeros.
+// sane: no corner position so large that its texel saturates.
+template <bool CLAMP>
 __device__ __forceinline__ bool slab_box(const SlabLaunch &L, const Corners &C, float sf, int &y0, int &y1,
                                          int &zlo, int &z1)
 {
+    constexpr float LIM = CLAMP ? 1.0e7f : 1.0e6f;
     int k1lo = 0x7fffffff, k1hi = -0x7fffffff, k2lo = 0x7fffffff, k2hi = -0x7fffffff;
     bool sane = true;
 #pragma unroll
     for (int k = 0; k < SLAB_NC; ++k) {
         const float q1 = fmaf(C.A1[k], sf, C.B1[k]), q2 = fmaf(C.A2[k], sf, C.B2[k]);
-        sane = sane && fabsf(q1) < 1.0e7f && fabsf(q2) < 1.0e7f;
-        const int k1 = min(max(floor_texel(q1), -2), L.n1), k2 = min(max(floor_texel(q2), -2), L.n2);
+        sane = sane && fabsf(q1) < LIM && fabsf(q2) < LIM;
+        int k1 = floor_texel(q1), k2 = floor_texel(q2);
+        if (CLAMP) {
+            k1 = min(max(k1, -2), L.n1);
+            k2 = min(max(k2, -2), L.n2);
+        }
         k1lo = min(k1lo, k1);
         k1hi = max(k1hi, k1);
         k2lo = min(k2lo, k2);
         k2hi = max(k2hi, k2);
     }
-    y0 = max(k1lo - 1, -2);
-    y1 = min(k1hi + 2, L.n1 + 1);
-    zlo = max(k2lo - 1, -2);
-    z1 = min(k2hi + 2, L.n2 + 1);
+    y0 = k1lo - 1;
+    y1 = k1hi + 2;
+    zlo = k2lo - 1;
+    z1 = k2hi + 2;
+    if (CLAMP) {
+        y0 = max(y0, -2);
+        y1 = min(y1, L.n1 + 1);
+        zlo = max(zlo, -2);
+        z1 = min(z1, L.n2 + 1);
+    }
     return sane;
 }
 
@@ -250,62 +282,71 @@ __device__ __noinline__ void slab_produce(const SlabLaunch &L, float2 *buf, uint
 {
     Corners C;
     slab_corners(L, lane, C);
-    const uint32_t sbuf = smem_u32(buf);
     const int nst = s_hi - s_lo + 1;
     unsigned long long n_staged = 0, n_global = 0;
     for (int b0 = 0; b0 < nst; b0 += 32) {
-        // lane k: the buffer box of slice s_lo + b0 + k
-        int y0, y1, zlo, z1;
-        const bool sane = slab_box(L, C, (float)(s_lo + b0 + lane), y0, y1, zlo, z1);
-        const int z0 = ((zlo + 2) & ~1) - 2;  // TMA: (z0 + 2) * 8 bytes on a 16-byte boundary
-        const int ny = y1 - y0 + 1, nz = z1 - z0 + 1;
-        const int sel = (!C.hull || !sane || ny > SLAB_BY || nz > SLAB_WB) ? -1 : (nz <= SLAB_WA ? 0 : 1);
-        const int pitch = sel == 0 ? SLAB_WA : SLAB_WB;
+        // lane k: the buffer box of slice s_lo + b0 + k; clamped to the zero
+        // border only when the rays' own extent does not fit a buffer
+        int y0, y1, zlo, z1, z0, ny, nz;
+        bool fit;
+        auto measure = [&](bool sane) {
+            z0 = ((zlo + 2) & ~1) - 2;  // TMA: (z0 + 2) * 8 bytes on a 16-byte boundary
+            ny = y1 - y0 + 1;
+            nz = z1 - z0 + 1;
+            fit = C.hull && sane && nz <= SLAB_WB &&
+                  ((ny + SLAB_BOX_Y - 1) / SLAB_BOX_Y) * SLAB_BOX_Y * (nz <= SLAB_WA ? SLAB_WA : SLAB_WB) <= SLAB_SLOT;
+        };
+        measure(slab_box<false>(L, C, (float)(s_lo + b0 + lane), y0, y1, zlo, z1));
+        const bool whole = fit;
+        if (!whole) measure(slab_box<true>(L, C, (float)(s_lo + b0 + lane), y0, y1, zlo, z1));
+        const int sel = !fit ? -1 : (nz <= SLAB_WA ? 0 : 1) + (whole ? 0 : 2);
+        const int pitch = (sel & 1) == 0 ? SLAB_WA : SLAB_WB;
         const int nby = (ny + SLAB_BOX_Y - 1) / SLAB_BOX_Y;
         const int cnt = min(32, nst - b0);
         if (lane < cnt) {
             if (sel >= 0) ++n_staged;
             else ++n_global;
         }
-        // the slices in order: each waits for its buffer, then its own lane
-        // writes the record and issues the loads
-        for (int k = 0; k < cnt; ++k) {
-            const int st = b0 + k;
-            const int slot = st % SLAB_STAGES;
+        // the stages in order: each waits for its buffers, then the lane of
+        // each of its slices writes the record and issues the loads
+        for (int k = 0; k < cnt; k += SLAB_PER) {
+            const int st = (b0 + k) / SLAB_PER;
+            const int stage = st % SLAB_STAGES;
             if (st >= SLAB_STAGES) {
                 const uint32_t par = (uint32_t)(((st / SLAB_STAGES) - 1) & 1);
-                if (!__all_sync(0xffffffffu, mbar_wait_bounded_sleep(&empty[slot], par, SLAB_WAIT))) {
+                if (!__all_sync(0xffffffffu, mbar_wait_bounded_sleep(&empty[stage], par, SLAB_WAIT))) {
                     if (lane == 0) atomicOr(&g_fp_slab_errors, (unsigned)B2T_DEVERR_WAIT_TIMEOUT);
-                    // the loads of the slices still in the buffers land first
+                    // the loads of the stages still in the buffers land first
                     for (int q = max(0, st - SLAB_STAGES); q < st; ++q)
                         (void)mbar_wait_bounded_sleep(&full[q % SLAB_STAGES], (uint32_t)((q / SLAB_STAGES) & 1),
                                                       SLAB_WAIT);
                     return;
                 }
             }
-            if (lane == k) {
+            if (lane >= k && lane < k + SLAB_PER) {
+                const int slot = stage * SLAB_PER + lane - k;
+                const bool load = sel >= 0 && lane < cnt;
                 SlabInfo r;
                 r.sel = sel;
-                r.rbase = (int)(0u - (uint32_t)(SPLIT_BITS + y0) * (uint32_t)(8 * pitch) -
-                                (uint32_t)(SPLIT_BITS + z0) * 8u);
+                r.rbase = (int)(smem_u32(buf) + (uint32_t)slot * (SLAB_SLOT * 8u) -
+                                (uint32_t)(SPLIT_BITS + y0) * (uint32_t)(8 * pitch) - (uint32_t)(SPLIT_BITS + z0) * 8u);
                 r.pad0 = r.pad1 = 0;
                 info[slot] = r;
-                if (sel >= 0) {
+                if (load) {
                     // the loads go out after the arrival, whose transaction
                     // count keeps the phase open until they land
-                    mbar_arrive_expect_tx(&full[slot], (uint32_t)(nby * SLAB_BOX_Y * pitch * sizeof(float2)));
+                    mbar_arrive_expect_tx(&full[stage], (uint32_t)(nby * SLAB_BOX_Y * pitch * sizeof(float2)));
                     float2 *dst = buf + (size_t)slot * SLAB_SLOT;
                     for (int by = 0; by < nby; ++by)
-                        tma_load_3d(dst + (size_t)(by * SLAB_BOX_Y) * pitch, &L.tmap[sel], z0 + 2,
-                                    y0 + 2 + by * SLAB_BOX_Y, s_lo + st, &full[slot]);
+                        tma_load_3d(dst + (size_t)(by * SLAB_BOX_Y) * pitch, &L.tmap[sel & 1], z0 + 2,
+                                    y0 + 2 + by * SLAB_BOX_Y, s_lo + b0 + lane, &full[stage]);
                 } else {
-                    mbar_arrive(&full[slot]);
+                    mbar_arrive(&full[stage]);
                 }
             }
             __syncwarp();
         }
     }
-    (void)sbuf;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         n_staged += __shfl_xor_sync(0xffffffffu, n_staged, o);
@@ -315,8 +356,9 @@ __device__ __noinline__ void slab_produce(const SlabLaunch &L, float2 *buf, uint
         atomicAdd(&g_fp_slab_slices[0], n_staged);
         atomicAdd(&g_fp_slab_slices[1], n_global);
     }
-    // the last slices' loads land before the warp leaves
-    for (int st = max(0, nst - SLAB_STAGES); st < nst; ++st)
+    // the last stages' loads land before the warp leaves
+    const int ns = (nst + SLAB_PER - 1) / SLAB_PER;
+    for (int st = max(0, ns - SLAB_STAGES); st < ns; ++st)
         (void)mbar_wait_bounded_sleep(&full[st % SLAB_STAGES], (uint32_t)((st / SLAB_STAGES) & 1), SLAB_WAIT);
 }
 
@@ -416,94 +458,125 @@ __device__ __forceinline__ void sample_global(const SlabLaunch &L, int s, float 
     }
 }
 
-// The CTA's slice range [s_lo, s_hi] and the warp's union [wlo, whi] and
-// intersection [ilo, ihi] of its rays' ranges.
+// The CTA's slice range [s_lo, s_hi] and the warp's union [wlo, whi] and (the
+// transpose) intersection [ilo, ihi] of its rays' ranges.
 struct Range {
     int s_lo, s_hi, wlo, whi, ilo, ihi;
 };
 
-// Slices [s0, s1] of a compute warp's pass (rows r < RE of each view): wait
-// for each slice's buffer, sample it (KIND 0: no ray of the warp samples
-// these slices, 1: some ray leaves the volume, texels clamped, 2: fast),
-// release it.  False when a wait gave up.
+// One slice of a compute warp's rays from the buffer of record I.
+template <int RE>
+__device__ __forceinline__ void slab_sample(const SlabLaunch &L, const SlabInfo &I, int s, float sf, Rays &R)
+{
+    const uint32_t rb = (uint32_t)I.rbase;
+    if (I.sel == 0) sample_smem<SLAB_WA, false, RE>(L, rb, sf, R);
+    else if (I.sel == 1) sample_smem<SLAB_WB, false, RE>(L, rb, sf, R);
+    else if (I.sel == 2) sample_smem<SLAB_WA, true, RE>(L, rb, sf, R);
+    else if (I.sel == 3) sample_smem<SLAB_WB, true, RE>(L, rb, sf, R);
+    else sample_global<RE>(L, s, sf, R);
+}
+
+// Stages [t0, t1) of a compute warp's pass (rows r < RE of each view): wait
+// for each stage's buffers, sample its slices (KIND 0: none is in the warp's
+// range [w0, w1], 1: some may be, 2: all are), release it.  False when a wait
+// gave up.
 template <int RE, int KIND>
-__device__ __forceinline__ bool slab_slices(const SlabLaunch &L, uint32_t sbase, uint64_t *full, uint64_t *empty,
-                                            const SlabInfo *info, int lane, int s0, int s1, int &slot,
+__device__ __forceinline__ bool slab_stages(const SlabLaunch &L, uint64_t *full, uint64_t *empty, const SlabInfo *info,
+                                            int lane, int s_lo, int t0, int t1, int w0, int w1, int &stage,
                                             uint32_t &par, Rays &R)
 {
-    float sf = (float)s0;
-    for (int s = s0; s <= s1; ++s, sf += 1.0f) {
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full[slot], par, SLAB_WAIT))) {
+    for (int t = t0; t < t1; ++t) {
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full[stage], par, SLAB_WAIT))) {
             if (lane == 0) atomicOr(&g_fp_slab_errors, (unsigned)B2T_DEVERR_WAIT_TIMEOUT);
             return false;
         }
-        if constexpr (KIND > 0) {
-            const SlabInfo I = info[slot];
-            const uint32_t rb = sbase + (uint32_t)slot * (SLAB_SLOT * 8u) + (uint32_t)I.rbase;
-            if (I.sel == 0) sample_smem<SLAB_WA, KIND == 1, RE>(L, rb, sf, R);
-            else if (I.sel == 1) sample_smem<SLAB_WB, KIND == 1, RE>(L, rb, sf, R);
-            else sample_global<RE>(L, s, sf, R);
+        if constexpr (KIND == 2) {
+            const float sf = (float)(s_lo + t * SLAB_PER);
+#pragma unroll
+            for (int i = 0; i < SLAB_PER; ++i)
+                slab_sample<RE>(L, info[stage * SLAB_PER + i], s_lo + t * SLAB_PER + i, sf + (float)i, R);
+        } else if constexpr (KIND == 1) {
+#pragma unroll 1
+            for (int i = 0; i < SLAB_PER; ++i) {
+                const int s = s_lo + t * SLAB_PER + i;
+                if (s >= w0 && s <= w1) slab_sample<RE>(L, info[stage * SLAB_PER + i], s, (float)s, R);
+            }
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[slot]);
-        if (++slot == SLAB_STAGES) {
-            slot = 0;
+        if (lane == 0) mbar_arrive(&empty[stage]);
+        if (++stage == SLAB_STAGES) {
+            stage = 0;
             par ^= 1u;
         }
     }
     return true;
 }
 
-// A compute warp's pass over the CTA's slices, split into the segments
-// where its sampling is the same for every slice (no per-slice range tests;
-// 137.0 -> 133.4 ms at 512^3 x 720, bit-identical).
+// A compute warp's pass over the CTA's slices: the stages before the warp's
+// range, its first, the whole ones, its last, the stages after it (no
+// per-slice range tests in the whole ones).
 template <int RE>
-__device__ __forceinline__ bool slab_consume(const SlabLaunch &L, const float2 *buf, uint64_t *full, uint64_t *empty,
+__device__ __forceinline__ bool slab_consume(const SlabLaunch &L, uint64_t *full, uint64_t *empty,
                                              const SlabInfo *info, int lane, const Range &rg, Rays &R)
 {
-    const uint32_t sbase = smem_u32(buf);
-    int slot = 0;
+    int stage = 0;
     uint32_t par = 0;
-    // the warp's slices in segments: none of its rays, clamped, fast, clamped, none
+    const int ns = rg.s_lo <= rg.s_hi ? (rg.s_hi - rg.s_lo) / SLAB_PER + 1 : 0;  // (0: no ray of the CTA meets the volume)
     const bool any = rg.wlo <= rg.whi;
     const int w0 = any ? rg.wlo : rg.s_hi + 1, w1 = any ? rg.whi : rg.s_hi;
-    const bool hasf = any && rg.ilo <= rg.ihi;
-    const int f0 = hasf ? max(rg.ilo, w0) : w1 + 1, f1 = hasf ? min(rg.ihi, w1) : w1;
-    if (!slab_slices<RE, 0>(L, sbase, full, empty, info, lane, rg.s_lo, w0 - 1, slot, par, R)) return false;
-    if (!slab_slices<RE, 1>(L, sbase, full, empty, info, lane, w0, f0 - 1, slot, par, R)) return false;
-    if (!slab_slices<RE, 2>(L, sbase, full, empty, info, lane, f0, f1, slot, par, R)) return false;
-    if (!slab_slices<RE, 1>(L, sbase, full, empty, info, lane, f1 + 1, w1, slot, par, R)) return false;
-    return slab_slices<RE, 0>(L, sbase, full, empty, info, lane, w1 + 1, rg.s_hi, slot, par, R);
+    // stages with a slice of the range: [ta, tb); with nothing else: [fa, fb)
+    const int ta = any ? (w0 - rg.s_lo) / SLAB_PER : ns, tb = any ? (w1 - rg.s_lo) / SLAB_PER + 1 : ns;
+    const int fa = min(tb, (w0 - rg.s_lo + SLAB_PER - 1) / SLAB_PER), fb = max(fa, (w1 + 1 - rg.s_lo) / SLAB_PER);
+    auto run = [&](auto kind, int t0, int t1) {
+        return slab_stages<RE, decltype(kind)::value>(L, full, empty, info, lane, rg.s_lo, t0, t1, w0, w1, stage, par, R);
+    };
+    if (!run(std::integral_constant<int, 0>{}, 0, ta)) return false;
+    if (!run(std::integral_constant<int, 1>{}, ta, any ? fa : ta)) return false;
+    if (any && !run(std::integral_constant<int, 2>{}, fa, fb)) return false;
+    if (any && !run(std::integral_constant<int, 1>{}, fb, tb)) return false;
+    return run(std::integral_constant<int, 0>{}, tb, ns);
 }
 
 // slab_consume for the rows in use, re in [1, RE]
 template <int RE>
-__device__ __forceinline__ bool slab_consume_rows(int re, const SlabLaunch &L, const float2 *buf, uint64_t *full,
-                                                  uint64_t *empty, const SlabInfo *info, int lane, const Range &rg,
+__device__ __forceinline__ bool slab_consume_rows(int re, const SlabLaunch &L, uint64_t *full, uint64_t *empty,
+                                                  const SlabInfo *info, int lane, const Range &rg,
                                                   Rays &R)
 {
     if constexpr (RE == 1) {
-        return slab_consume<1>(L, buf, full, empty, info, lane, rg, R);
+        return slab_consume<1>(L, full, empty, info, lane, rg, R);
     } else {
-        if (re >= RE) return slab_consume<RE>(L, buf, full, empty, info, lane, rg, R);
-        return slab_consume_rows<RE - 1>(re, L, buf, full, empty, info, lane, rg, R);
+        if (re >= RE) return slab_consume<RE>(L, full, empty, info, lane, rg, R);
+        return slab_consume_rows<RE - 1>(re, L, full, empty, info, lane, rg, R);
     }
 }
 
+__device__ __forceinline__ float to_f32(float v) { return v; }
+__device__ __forceinline__ float to_f32(__half v) { return __half2float(v); }
+__device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
+template <typename T> __device__ __forceinline__ T from_f32(float v);
+template <> __device__ __forceinline__ float from_f32<float>(float v) { return v; }
+template <> __device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
+template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+
+// T: the projections' storage type (the slab copy holds FP32 for every type,
+// so 16-bit data are sampled exactly as FP32 data of the same values and
+// rounded once, at the store).
+template <typename T>
 __global__ void __launch_bounds__(SLAB_THREADS, 2) fp3d_slab_kernel(const __grid_constant__ SlabLaunch L)
 {
     extern __shared__ __align__(1024) unsigned char smraw[];
     float2 *buf = reinterpret_cast<float2 *>(smraw);
-    uint64_t *full = reinterpret_cast<uint64_t *>(smraw + (size_t)SLAB_STAGES * SLAB_SLOT * sizeof(float2));
+    uint64_t *full = reinterpret_cast<uint64_t *>(smraw + (size_t)SLAB_SLOTS * SLAB_SLOT * sizeof(float2));
     uint64_t *empty = full + SLAB_STAGES;
     SlabInfo *info = reinterpret_cast<SlabInfo *>(empty + SLAB_STAGES);
-    int *range = reinterpret_cast<int *>(info + SLAB_STAGES);
+    int *range = reinterpret_cast<int *>(info + SLAB_SLOTS);
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         for (int k = 0; k < SLAB_STAGES; ++k) {
-            mbar_init(&full[k], 1);
+            mbar_init(&full[k], SLAB_PER);
             mbar_init(&empty[k], SLAB_WARPS);
         }
         range[0] = 0x7fffffff;
@@ -517,16 +590,16 @@ __global__ void __launch_bounds__(SLAB_THREADS, 2) fp3d_slab_kernel(const __grid
     // ---- ray set-up (compute warps): column `warp`, both views, SLAB_R rows per lane
     const int u_raw = (int)blockIdx.y * SLAB_U + warp;
     Rays R;
-    int wlo = 1, whi = 0, ilo = 1, ihi = 0;  // union and intersection of the warp's ray ranges
+    int wlo = 1, whi = 0;  // union of the warp's ray ranges
     if (warp < SLAB_WARPS) {
         const float uu = det_uu(L, u_raw);
-        int lo_u = 0x7fffffff, hi_u = -0x7fffffff, lo_i = -0x7fffffff, hi_i = 0x7fffffff;
+        int lo_u = 0x7fffffff, hi_u = -0x7fffffff;
 #pragma unroll
         for (int w = 0; w < SLAB_W; ++w) {
             const FPView &V = L.views[min((int)blockIdx.x * SLAB_W + w, L.nviews - 1)];
 #pragma unroll
             for (int r = 0; r < SLAB_R; ++r) {
-                const int v = (int)blockIdx.z * SLAB_ROWS + lane + 32 * r;
+                const int v = (int)blockIdx.z * L.rows + lane + 32 * r;
                 float a1, b1;
                 ray_setup(V, uu, det_vv(L, v), a1, b1, R.A2[w][r], R.B2h[w][r]);
                 // the same for every row: a column's rays share the in-plane position
@@ -536,18 +609,14 @@ __global__ void __launch_bounds__(SLAB_THREADS, 2) fp3d_slab_kernel(const __grid
                 int lo = 0, hi = L.n0 - 1;
                 clip_axis(a1, b1, L.n1, L.n0, lo, hi);
                 clip_axis(R.A2[w][r], R.B2h[w][r], L.n2, L.n0, lo, hi);
-                if (lo <= hi) {
+                if (lo <= hi && 32 * r < L.rows) {
                     lo_u = min(lo_u, lo);
                     hi_u = max(hi_u, hi);
                 }
-                lo_i = max(lo_i, lo);
-                hi_i = min(hi_i, hi);
             }
         }
         wlo = warp_min(lo_u);
         whi = warp_max(hi_u);
-        ilo = warp_max(lo_i);
-        ihi = warp_min(hi_i);
         if (lane == 0 && wlo <= whi) {
             atomicMin(&range[0], wlo);
             atomicMax(&range[1], whi);
@@ -563,10 +632,10 @@ __global__ void __launch_bounds__(SLAB_THREADS, 2) fp3d_slab_kernel(const __grid
 
     // ---- compute warps: the rows in use (the last row block of the
     // detector may hold fewer than SLAB_ROWS)
-    const int re = min(SLAB_R, (L.nv - (int)blockIdx.z * SLAB_ROWS + 31) >> 5);
-    const Range rg{s_lo, s_hi, wlo, whi, ilo, ihi};
+    const int re = min(L.rows, L.nv - (int)blockIdx.z * L.rows + 31) >> 5;
+    const Range rg{s_lo, s_hi, wlo, whi, 0, 0};
     bool ok;
-    ok = slab_consume_rows<SLAB_R>(re, L, buf, full, empty, info, lane, rg, R);
+    ok = slab_consume_rows<SLAB_R>(re, L, full, empty, info, lane, rg, R);
     if (!ok || u_raw >= L.nu) return;
     // ---- results
 #pragma unroll
@@ -576,14 +645,14 @@ __global__ void __launch_bounds__(SLAB_THREADS, 2) fp3d_slab_kernel(const __grid
         const int a = L.views[vi].a;
 #pragma unroll
         for (int r = 0; r < SLAB_R; ++r) {
-            const int v = (int)blockIdx.z * SLAB_ROWS + lane + 32 * r;
-            if (v >= L.nv) continue;
+            const int v = (int)blockIdx.z * L.rows + lane + 32 * r;
+            if (v >= L.nv || 32 * r >= L.rows) continue;
             const float sc =
                 sqrtf(fmaf(R.A1[w] * R.A1[w], L.f1, fmaf(R.A2[w][r] * R.A2[w][r], L.f2, 1.0f))) * L.mul;
-            float *out = static_cast<float *>(L.proj) + ((size_t)v * L.na + a) * L.proj_pitch + u_raw;
+            T *out = static_cast<T *>(L.proj) + ((size_t)v * L.na + a) * L.proj_pitch + u_raw;
             float val = fmaf(R.acc[w][r], sc, 0.0f);
-            if (L.accumulate) val += *out;
-            *out = val;
+            if (L.accumulate) val += to_f32(*out);
+            *out = from_f32<T>(val);
         }
     }
 }
@@ -624,7 +693,8 @@ __global__ void __launch_bounds__(SLAB_THREADS, 2) fp3d_slab_kernel(const __grid
 constexpr int MT_STAGES = 4;              // slice boxes in flight
 constexpr int MT_LAG = 2;                 // slices between a box's last scatter and its flush
 constexpr int MT_WA = 96, MT_WB = 160;    // box widths (floats): a box's row pitch
-constexpr int MT_SLOT = SLAB_BY * MT_WB;  // floats per box
+constexpr int MT_BY = 24;                 // box rows
+constexpr int MT_SLOT = MT_BY * MT_WB;  // floats per box
 static_assert(MT_LAG >= 1 && MT_LAG < MT_STAGES, "a box is flushed before its slot comes round again");
 static_assert((MT_WA * 4 * SLAB_BOX_Y) % 128 == 0 && (MT_WB * 4 * SLAB_BOX_Y) % 128 == 0,
               "TMA boxes start on 128-byte boundaries of a slot");
@@ -782,10 +852,10 @@ __device__ __noinline__ void mt_produce(const SlabLaunch &L, float *buf, uint64_
     for (int b0 = 0; b0 < nst && ok; b0 += 32) {
         // lane k: the box of slice s_lo + b0 + k
         int y0, y1, zlo, z1;
-        const bool sane = slab_box(L, C, (float)(s_lo + b0 + lane), y0, y1, zlo, z1);
+        const bool sane = slab_box<true>(L, C, (float)(s_lo + b0 + lane), y0, y1, zlo, z1);
         const int z0 = ((zlo + 2) & ~3) - 2;  // TMA: (z0 + 2) * 4 bytes on a 16-byte boundary
         const int ny = y1 - y0 + 1, nz = z1 - z0 + 1;
-        const int sel_l = (!C.hull || !sane || ny > SLAB_BY || nz > MT_WB) ? -1 : (nz <= MT_WA ? 0 : 1);
+        const int sel_l = (!C.hull || !sane || ny > MT_BY || nz > MT_WB) ? -1 : (nz <= MT_WA ? 0 : 1);
         const int nby_l = (ny + SLAB_BOX_Y - 1) / SLAB_BOX_Y;
         const int cnt = min(32, nst - b0);
         if (lane < cnt) {
@@ -991,31 +1061,33 @@ __global__ void __launch_bounds__(SLAB_THREADS, 2) bp3d_slab_matched_kernel(cons
 }
 
 // Slab copy of marching axis dir (0: slices along x, in-plane axis y; 1:
-// slices along y, in-plane axis x) as z-pairs: texel (s, k1, k2) holds
-// (v[k2], v[k2 + 1] - v[k2]) at (s * py + k1 + 2) * pz + k2 + 2, written for
-// k1 in [0, n1) and k2 in [-1, n2 - 1] (the pair below the volume carries
-// v[0] as its difference); everything else stays zero from a memset.  A CTA
-// transposes a (z, x) tile of one y plane through shared memory.
-__global__ void __launch_bounds__(256) build_slab_copy(const float *__restrict__ vol, size_t pitch, int nx, int ny,
+// slices along y, in-plane axis x) as z-pairs of FP32: texel (s, k1, k2) holds
+// (v[k2], v[k2 + 1] - v[k2]) at (s * py + k1 + 2) * pz + k2 + 2, zero texels
+// outside the volume, every cell of the copy written (no clearing pass).  A
+// CTA transposes a (z, x) tile of one y plane through shared memory; border
+// planes and columns of the in-plane axis are tiles outside the volume.
+template <typename T>
+__global__ void __launch_bounds__(256) build_slab_copy(const T *__restrict__ vol, size_t pitch, int nx, int ny,
                                                        int nz, int dir, long long py, long long pz,
                                                        float2 *__restrict__ out)
 {
-    __shared__ float t[34][33];  // t[i][xi] = v(z0 - 1 + i, y, x0 + xi), zero outside the volume
-    const int z0 = blockIdx.x * 32, x0 = blockIdx.y * 32, y = blockIdx.z;
+    __shared__ float t[33][33];  // t[i][xi] = v(z0 + i, y, x0 + xi), zero outside the volume
+    const int z0 = (int)blockIdx.x * 32 - 2;
+    const int x0 = (int)blockIdx.y * 32 - (dir == 0 ? 0 : 2), y = (int)blockIdx.z - (dir == 0 ? 2 : 0);
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int i = ty; i < 34; i += 8) {
-        const int z = z0 - 1 + i, x = x0 + tx;
-        t[i][tx] = (z >= 0 && z < nz && x < nx) ? __ldg(vol + ((size_t)z * ny + y) * pitch + x) : 0.0f;
+    for (int i = ty; i < 33; i += 8) {
+        const int z = z0 + i, x = x0 + tx;
+        const bool in = (unsigned)z < (unsigned)nz && (unsigned)x < (unsigned)nx && (unsigned)y < (unsigned)ny;
+        t[i][tx] = in ? to_f32(vol[((size_t)z * ny + y) * pitch + x]) : 0.0f;
     }
     __syncthreads();
+    const int j = (int)blockIdx.x * 32 + tx;
+    if (j >= pz) return;
     for (int xi = ty; xi < 32; xi += 8) {
         const int x = x0 + xi;
-        if (x >= nx) continue;
+        if (x >= nx + (dir == 0 ? 0 : 2)) break;
         const long long s = (dir == 0) ? x : y, k1 = (dir == 0) ? y : x;
-        float2 *row = out + (s * py + k1 + 2) * pz + 2;
-        const int z = z0 + tx;
-        if (z < nz) row[z] = make_float2(t[tx + 1][xi], t[tx + 2][xi] - t[tx + 1][xi]);
-        if (z0 == 0 && tx == 0) row[-1] = make_float2(0.0f, t[1][xi]);
+        out[(s * py + k1 + 2) * pz + j] = make_float2(t[tx][xi], t[tx + 1][xi] - t[tx][xi]);
     }
 }
 
@@ -1054,10 +1126,11 @@ b2t_status fp_slab_errors(uint32_t *flags)
     return B2T_OK;
 }
 
-bool fp_slab_eligible(const b2t_geom3d *g, const b2t_params3d *p, int32_t dtype, int dir, const std::vector<int> &dirs)
+bool fp_slab_eligible(const b2t_geom3d *g, const b2t_params3d *p, int dir, const std::vector<int> &dirs)
 {
-    if (!slab_enabled() || dtype != B2T_F32 || dir > 1 || p->det_supersample != 1) return false;
+    if (!slab_enabled() || dir > 1 || p->det_supersample != 1) return false;
     const b2t_dims3d &d = g->dims;
+    if (d.vol_y + 4 > 65535) return false;  // (the copy's grid)
     for (uint32_t a = 0; a < d.angles; ++a) {
         if (dirs[a] != dir) continue;
         FPView w;
@@ -1073,21 +1146,36 @@ size_t fp_slab_copy_bytes(const b2t_dims3d &d, int dir)
     return n0 * (n1 + 4) * (size_t)slab_pz(d) * sizeof(float2);
 }
 
-b2t_status fp_slab_build(const b2t_dims3d &d, const float *vol, size_t vol_pitch, int dir, void *copy,
+b2t_status fp_slab_build(const b2t_dims3d &d, const void *vol, size_t vol_pitch, int32_t dtype, int dir, void *copy,
                          cudaStream_t s)
 {
-    const long long n1 = dir == 0 ? d.vol_y : d.vol_x;
-    B2T_CUDA_TRY(cudaMemsetAsync(copy, 0, fp_slab_copy_bytes(d, dir), s), "slab copy clear");
-    dim3 grid((d.vol_z + 31) / 32, (d.vol_x + 31) / 32, d.vol_y);
-    build_slab_copy<<<grid, 256, 0, s>>>(vol, vol_pitch, d.vol_x, d.vol_y, d.vol_z, dir, n1 + 4, slab_pz(d),
-                                         static_cast<float2 *>(copy));
+    const long long py = (dir == 0 ? d.vol_y : d.vol_x) + 4, pz = slab_pz(d);
+    const unsigned ex = d.vol_x + (dir == 0 ? 0 : 4), ey = d.vol_y + (dir == 0 ? 4 : 0);
+    const dim3 grid((unsigned)((pz + 31) / 32), (ex + 31) / 32, ey);
+    float2 *out = static_cast<float2 *>(copy);
+    auto build = [&](auto *v) {
+        build_slab_copy<<<grid, 256, 0, s>>>(v, vol_pitch, (int)d.vol_x, (int)d.vol_y, (int)d.vol_z, dir, py, pz, out);
+    };
+    if (dtype == B2T_F32) build(static_cast<const float *>(vol));
+    else if (dtype == B2T_F16) build(static_cast<const __half *>(vol));
+    else build(static_cast<const __nv_bfloat16 *>(vol));
     count_launches(1);
     B2T_CUDA_TRY(cudaGetLastError(), "slab copy launch");
     return B2T_OK;
 }
 
+template <typename T>
+static cudaError_t launch_slab(const SlabLaunch &L, dim3 grid, size_t smem, cudaStream_t s)
+{
+    const cudaError_t e =
+        cudaFuncSetAttribute(fp3d_slab_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    fp3d_slab_kernel<T><<<grid, SLAB_THREADS, smem, s>>>(L);
+    return cudaGetLastError();
+}
+
 b2t_status fp_slab_project(const b2t_geom3d *g, const b2t_params3d *p, const void *copy, int dir, void *proj,
-                           size_t proj_pitch, int32_t mode, const std::vector<int> &dirs, cudaStream_t s)
+                           size_t proj_pitch, int32_t dtype, int32_t mode, const std::vector<int> &dirs, cudaStream_t s)
 {
     const b2t_dims3d &d = g->dims;
     SlabLaunch *Lp = new SlabLaunch;
@@ -1116,18 +1204,15 @@ b2t_status fp_slab_project(const b2t_geom3d *g, const b2t_params3d *p, const voi
     L.nv = d.det_v;
     L.na = d.angles;
     L.accumulate = (mode == B2T_MODE_ADD) ? 1 : 0;
+    // the fewest row blocks, of equal height
+    const int blocks = (int)((d.det_v + SLAB_ROWS - 1) / SLAB_ROWS);
+    L.rows = 32 * (((int)d.det_v + 32 * blocks - 1) / (32 * blocks));
     fp_scale(g->kind, dir, g->vol_scale, false, p->output_scale, L.f1, L.f2, L.mul);
     std::vector<int> views;
     for (uint32_t a = 0; a < d.angles; ++a)
         if (dirs[a] == dir) views.push_back((int)a);
-    const size_t smem = (size_t)SLAB_STAGES * SLAB_SLOT * sizeof(float2) +
-                        SLAB_STAGES * (2 * sizeof(uint64_t) + sizeof(SlabInfo)) + 2 * sizeof(int);
-    static bool attr_set = false;
-    if (!attr_set) {
-        B2T_CUDA_TRY(cudaFuncSetAttribute(fp3d_slab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                     "slab FP shared memory attribute");
-        attr_set = true;
-    }
+    const size_t smem = (size_t)SLAB_SLOTS * SLAB_SLOT * sizeof(float2) + SLAB_STAGES * 2 * sizeof(uint64_t) +
+                        SLAB_SLOTS * sizeof(SlabInfo) + 2 * sizeof(int);
     for (size_t c0 = 0; c0 < views.size() && st == B2T_OK; c0 += SLAB_MAX_VIEWS) {
         const size_t cn = std::min(views.size() - c0, (size_t)SLAB_MAX_VIEWS);
         L.nviews = (int)cn;
@@ -1136,11 +1221,12 @@ b2t_status fp_slab_project(const b2t_geom3d *g, const b2t_params3d *p, const voi
             L.views[i].a = views[c0 + i];
         }
         dim3 grid((unsigned)((cn + SLAB_W - 1) / SLAB_W), (d.det_u + SLAB_U - 1) / SLAB_U,
-                  (d.det_v + SLAB_ROWS - 1) / SLAB_ROWS);
-        fp3d_slab_kernel<<<grid, SLAB_THREADS, smem, s>>>(L);
+                  (d.det_v + (unsigned)L.rows - 1) / (unsigned)L.rows);
+        const cudaError_t e = dtype == B2T_F32   ? launch_slab<float>(L, grid, smem, s)
+                              : dtype == B2T_F16 ? launch_slab<__half>(L, grid, smem, s)
+                                                 : launch_slab<__nv_bfloat16>(L, grid, smem, s);
         count_launches(1);
         g_slab_launches.fetch_add(1);
-        cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) st = cuda_fail(e, "fp3d_slab_kernel launch");
     }
     delete Lp;
@@ -1170,7 +1256,7 @@ bool matched_slab_eligible(const b2t_geom3d *g, const b2t_params3d *p, int dir, 
 void matched_slab_dims(const b2t_dims3d &d, int dir, long long &ay, long long &az)
 {
     // room for a whole box past the far border: no TMA reduce leaves the array
-    ay = (long long)(dir == 0 ? d.vol_y : d.vol_x) + 4 + SLAB_BY;
+    ay = (long long)(dir == 0 ? d.vol_y : d.vol_x) + 4 + MT_BY;
     az = ((long long)d.vol_z + 4 + MT_WB + 3) & ~3ll;
 }
 
@@ -1227,6 +1313,7 @@ b2t_status matched_slab_scatter(const b2t_geom3d *g, const b2t_params3d *p, cons
     L.nv = d.det_v;
     L.na = d.angles;
     L.accumulate = 0;
+    L.rows = SLAB_ROWS;
     fp_scale(g->kind, dir, g->vol_scale, false, p->output_scale, L.f1, L.f2, L.mul);
     std::vector<int> views;
     for (uint32_t a = 0; a < d.angles; ++a)

@@ -151,14 +151,14 @@ b2t_status fp3d_cells_build(const b2t_geom3d *g, const b2t_params3d *p, const vo
                             int32_t dtype, const bool need[3], cudaStream_t s, FPCells &c);
 
 // TMA-staged slab forward projector (fp3d_slab.cu) for x- and y-major views
-// whose rays share the in-plane position along a detector column: FP32,
-// no detector supersampling.
-bool fp_slab_eligible(const b2t_geom3d *g, const b2t_params3d *p, int32_t dtype, int dir, const std::vector<int> &dirs);
+// whose rays share the in-plane position along a detector column, any storage
+// type, no detector supersampling.
+bool fp_slab_eligible(const b2t_geom3d *g, const b2t_params3d *p, int dir, const std::vector<int> &dirs);
 size_t fp_slab_copy_bytes(const b2t_dims3d &d, int dir);
-b2t_status fp_slab_build(const b2t_dims3d &d, const float *vol, size_t vol_pitch, int dir, void *copy,
+b2t_status fp_slab_build(const b2t_dims3d &d, const void *vol, size_t vol_pitch, int32_t dtype, int dir, void *copy,
                          cudaStream_t s);
 b2t_status fp_slab_project(const b2t_geom3d *g, const b2t_params3d *p, const void *copy, int dir, void *proj,
-                           size_t proj_pitch, int32_t mode, const std::vector<int> &dirs, cudaStream_t s);
+                           size_t proj_pitch, int32_t dtype, int32_t mode, const std::vector<int> &dirs, cudaStream_t s);
 b2t_status fp_slab_errors(uint32_t *flags);
 b2t_status fp_path_stats_impl(uint64_t *stats);
 unsigned long long fp_cell_launches_take();
