@@ -66,12 +66,8 @@ __global__ void sirt_update_kernel(float *__restrict__ x, const float *__restric
                                    const float *__restrict__ min_mask, const float *__restrict__ max_mask)
 {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        float v = fmaf(w[i], d[i], x[i]);
-        if (use_min && v < vmin) v = vmin;
-        if (use_max && v > vmax) v = vmax;
-        if (min_mask && v < min_mask[i]) v = min_mask[i];
-        if (max_mask && v > max_mask[i]) v = max_mask[i];
-        x[i] = v;
+        x[i] = sirt_clamp(fmaf(w[i], d[i], x[i]), use_min, vmin, use_max, vmax, min_mask ? min_mask + i : nullptr,
+                          max_mask ? max_mask + i : nullptr);
     }
 }
 
@@ -180,6 +176,14 @@ struct Operator {
     virtual b2t_status fp(const float *vol, float *proj, float scale, int mode, cudaStream_t s) = 0;
     // vol (=|+=) scale * B proj
     virtual b2t_status bp(const float *proj, float *vol, float scale, int mode, cudaStream_t s) = 0;
+    // r = (b - A vol) w and x = clamp(x + w B proj) in the projection's own
+    // launch; B2T_ERR_UNSUPPORTED or B2T_ERR_NO_MEMORY: not here, the caller
+    // runs the projection and the element-wise pass
+    virtual b2t_status fp_residual(const float *, const float *, const float *, float *, cudaStream_t)
+    {
+        return B2T_ERR_UNSUPPORTED;
+    }
+    virtual b2t_status bp_update(const float *, const SirtUpdate2D &, cudaStream_t) { return B2T_ERR_UNSUPPORTED; }
     // chunk tables when the operator is a batch of independent problems
     virtual const SegTable *segments(bool vol) const { return nullptr; }
     size_t nvol = 0, nproj = 0;
@@ -259,6 +263,15 @@ struct Op2D : Operator {
         b2t_geom2d q = g;
         q.output_scale *= scale;
         return bp2d_impl(&q, pix_ss, 0, proj, 0, vol, 0, mode, s);
+    }
+    b2t_status fp_residual(const float *vol, const float *b, const float *w, float *r, cudaStream_t s) override
+    {
+        return fp2d_lines(&g, det_ss, vol, g.dims.vol_width, r, g.dims.dets, B2T_MODE_SET, b, w, s);
+    }
+    b2t_status bp_update(const float *proj, const SirtUpdate2D &u, cudaStream_t s) override
+    {
+        if (pix_ss != 1 || g.dims.angles > (uint32_t)BP2D_MAX_VIEWS) return B2T_ERR_UNSUPPORTED;
+        return bp2d_lines(&g, 0, proj, g.dims.dets, nullptr, g.dims.vol_width, B2T_MODE_SET, &u, s);
     }
 };
 
@@ -433,9 +446,21 @@ struct Algo {
         b2t_status st;
         const float *xv = masked(vol, tmpVol.as<float>(), s, st);
         B2T_TRY(st);
-        B2T_TRY(op->fp(xv, tmpProj.as<float>(), 1.0f, B2T_MODE_SET, s));
-        residual_weight_kernel<<<ew_blocks(np()), EW_THREADS, 0, s>>>(tmpProj.as<float>(), sino, lineW.as<float>(), np());
-        B2T_TRY(ew(cudaGetLastError(), "SIRT residual"));
+        auto elsewhere = [](b2t_status r) { return r == B2T_ERR_UNSUPPORTED || r == B2T_ERR_NO_MEMORY; };
+        st = op->fp_residual(xv, sino, lineW.as<float>(), tmpProj.as<float>(), s);
+        if (elsewhere(st)) {
+            clear_error();
+            B2T_TRY(op->fp(xv, tmpProj.as<float>(), 1.0f, B2T_MODE_SET, s));
+            residual_weight_kernel<<<ew_blocks(np()), EW_THREADS, 0, s>>>(tmpProj.as<float>(), sino, lineW.as<float>(),
+                                                                          np());
+            st = ew(cudaGetLastError(), "SIRT residual");
+        }
+        B2T_TRY(st);
+        const SirtUpdate2D u{vol, pixW.as<float>(), opt.use_min, opt.use_max, opt.min_value, opt.max_value,
+                             opt.min_mask, opt.max_mask};
+        st = op->bp_update(tmpProj.as<float>(), u, s);
+        if (!elsewhere(st)) return st;
+        clear_error();
         B2T_TRY(op->bp(tmpProj.as<float>(), tmpVol.as<float>(), 1.0f, B2T_MODE_SET, s));
         sirt_update_kernel<<<ew_blocks(nv()), EW_THREADS, 0, s>>>(
             vol, pixW.as<float>(), tmpVol.as<float>(), nv(), opt.use_min, opt.min_value, opt.use_max, opt.max_value,

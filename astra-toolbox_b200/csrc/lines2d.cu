@@ -25,8 +25,8 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <memory>
 #include <type_traits>
-#include <vector>
 
 #include "b2t_internal.h"
 #include "f32x2.cuh"
@@ -117,6 +117,7 @@ struct FP2DLinesLaunch {
     long long sino_pitch;
     int W, H, ndet, rays, accumulate, a0, nviews;
     float out_scale;
+    const float *res_b, *res_w;  // SIRT's residual in place of the projection: (b - A x) w
     union {
         ParFPView par[FP2D_MAX_VIEWS];
         b2t_view2d fan[FP2D_MAX_VIEWS];
@@ -326,8 +327,9 @@ __global__ void __launch_bounds__(LINES_THREADS) fp2d_lines_kernel(const __grid_
         const int det = det0 + 8 * j;
         if (det >= L.ndet) continue;
         if constexpr (KIND == B2T_GEOM_PAR2D) acc[j] = __fmul_rn(acc[j], L.par[vi].corr / (float)R);
-        float *out = L.sino + (long long)(L.a0 + vi) * L.sino_pitch + det;
-        *out = L.accumulate ? *out + acc[j] : acc[j];
+        const long long i = (long long)(L.a0 + vi) * L.sino_pitch + det;
+        if (L.res_w) L.sino[i] = (L.res_b[i] - acc[j]) * L.res_w[i];
+        else L.sino[i] = L.accumulate ? L.sino[i] + acc[j] : acc[j];
     }
 }
 
@@ -343,6 +345,7 @@ struct BP2DLinesLaunch {
     int W, H, ndet, fbp, nviews, accumulate;
     int win;  // pairs per staged row
     float out_scale;
+    SirtUpdate2D upd;  // x set: SIRT's update in place of the backprojection
     BPView2D views[BP2D_MAX_VIEWS];  // parallel: c[2] less 1/2
 };
 
@@ -570,8 +573,15 @@ __global__ void __launch_bounds__(LINES_THREADS) bp2d_lines_kernel(const __grid_
     }
     auto store = [&](int px, int py, float t) {
         if (px >= L.W || py >= L.H) return;
-        float *o = L.vol + (long long)py * L.vol_pitch + px;
         const float r = __fmul_rn(t, L.out_scale);
+        const long long i = (long long)py * L.vol_pitch + px;
+        if (L.upd.x) {
+            const SirtUpdate2D &U = L.upd;
+            U.x[i] = sirt_clamp(fmaf(U.w[i], r, U.x[i]), U.use_min, U.min_value, U.use_max, U.max_value,
+                                U.min_mask ? U.min_mask + i : nullptr, U.max_mask ? U.max_mask + i : nullptr);
+            return;
+        }
+        float *o = L.vol + i;
         *o = L.accumulate ? *o + r : r;
     };
     if constexpr (WS > 1) {
@@ -678,7 +688,7 @@ cudaError_t launch_bp(BP2DLinesLaunch &L, float step, cudaStream_t s)
 }  // namespace
 
 b2t_status fp2d_lines(const b2t_geom2d *g, uint32_t det_supersample, const float *vol, size_t vol_pitch, float *sino,
-                      size_t sino_pitch, int32_t mode, cudaStream_t s)
+                      size_t sino_pitch, int32_t mode, const float *res_b, const float *res_w, cudaStream_t s)
 {
     const b2t_dims2d &d = g->dims;
     // which lines the rays march over: a parallel view's rays share the
@@ -694,8 +704,10 @@ b2t_status fp2d_lines(const b2t_geom2d *g, uint32_t det_supersample, const float
     if (cols) lines_bytes(d.vol_width, d.vol_height, total);
     Scratch sc;
     B2T_TRY(sc.alloc(total, s, "b2t_fp2d scratch (line copy)"));
-    std::vector<FP2DLinesLaunch> keep(1);
-    FP2DLinesLaunch &L = keep[0];
+    const std::unique_ptr<FP2DLinesLaunch> keep(new FP2DLinesLaunch);
+    FP2DLinesLaunch &L = *keep;
+    L.res_b = res_b;
+    L.res_w = res_w;
     L.pitch[0] = (d.vol_width + 2 * LINE_BORDER) * (uint32_t)sizeof(float2);
     L.pitch[1] = (d.vol_height + 2 * LINE_BORDER) * (uint32_t)sizeof(float2);
     L.line0[0] = sc.as<char>() + LINE_BORDER * sizeof(float2);
@@ -730,11 +742,12 @@ b2t_status fp2d_lines(const b2t_geom2d *g, uint32_t det_supersample, const float
 }
 
 b2t_status bp2d_lines(const b2t_geom2d *g, int32_t fbp_weight, const float *sino, size_t sino_pitch, float *vol,
-                      size_t vol_pitch, int32_t mode, cudaStream_t s)
+                      size_t vol_pitch, int32_t mode, const SirtUpdate2D *update, cudaStream_t s)
 {
     const b2t_dims2d &d = g->dims;
-    std::vector<BP2DLinesLaunch> keep(1);
-    BP2DLinesLaunch &L = keep[0];
+    const std::unique_ptr<BP2DLinesLaunch> keep(new BP2DLinesLaunch);
+    BP2DLinesLaunch &L = *keep;
+    L.upd = update ? *update : SirtUpdate2D{};
     L.sino_pitch = (long long)sino_pitch;
     L.vol = vol;
     L.vol_pitch = (long long)vol_pitch;

@@ -53,14 +53,38 @@ struct BP2DLaunch {
     BPView2D views[BP2D_MAX_VIEWS];
 };
 
-// 2D projection from line copies (lines2d.cu): a copy of the image's rows
-// and columns (FP) or of the sinogram's rows (BP) as pairs of neighbouring
-// texels inside a zero border.  B2T_ERR_NO_MEMORY when the copy does not fit
-// (its scratch, or 32-bit offsets): the callers then read the data directly.
+// SIRT's volume update x = clamp(x + w B r) on tightly packed images.
+struct SirtUpdate2D {
+    float *x = nullptr;
+    const float *w = nullptr;
+    int use_min = 0, use_max = 0;
+    float min_value = 0.0f, max_value = 0.0f;
+    const float *min_mask = nullptr, *max_mask = nullptr;
+};
+
+#ifdef __CUDACC__
+// v clamped to the scalar bounds and the pixel's own ones (null: none).
+__device__ __forceinline__ float sirt_clamp(float v, int use_min, float vmin, int use_max, float vmax,
+                                            const float *min_mask, const float *max_mask)
+{
+    if (use_min && v < vmin) v = vmin;
+    if (use_max && v > vmax) v = vmax;
+    if (min_mask && v < *min_mask) v = *min_mask;
+    if (max_mask && v > *max_mask) v = *max_mask;
+    return v;
+}
+#endif
+
+// 2D projection from lines of texel pairs (lines2d.cu).  The FP copies the
+// image's lines once; B2T_ERR_NO_MEMORY when the scratch does not fit: the
+// caller then reads the image directly.  With res_w, the FP stores SIRT's
+// residual (res_b - A vol) res_w (packed like sino) instead of A vol.  With
+// update, the BP applies SIRT's update instead of storing to vol (views of a
+// single launch only: at most BP2D_MAX_VIEWS).
 b2t_status fp2d_lines(const b2t_geom2d *g, uint32_t det_supersample, const float *vol, size_t vol_pitch, float *sino,
-                      size_t sino_pitch, int32_t mode, cudaStream_t s);
+                      size_t sino_pitch, int32_t mode, const float *res_b, const float *res_w, cudaStream_t s);
 b2t_status bp2d_lines(const b2t_geom2d *g, int32_t fbp_weight, const float *sino, size_t sino_pitch, float *vol,
-                      size_t vol_pitch, int32_t mode, cudaStream_t s);
+                      size_t vol_pitch, int32_t mode, const SirtUpdate2D *update, cudaStream_t s);
 
 b2t_status validate2d(const b2t_geom2d *g, const char *who);
 void par_fp_view(const b2t_view2d &p, const b2t_dims2d &d, float out_scale, ParFPView &o);
