@@ -84,11 +84,13 @@ void par_fp_view(const b2t_view2d &p, const b2t_dims2d &d, float out_scale, ParF
     double t = (ux * rx + uy * ry) / (rx * rx + ry * ry);
     ux -= t * rx;
     uy -= t * ry;
-    const float fAngle = (float)atan2(uy, ux);
     const double norm2 = uy * uy + ux * ux;
     const float fDetSize = (float)sqrt(norm2);
     const float fOffset = (float)(-0.5 * d.dets - (p.det_s[1] * uy + p.det_s[0] * ux) / norm2);
-    const double c = cos((double)fAngle), s = sin((double)fAngle);
+    // cosine and sine of the detector's direction, from the vector itself: the
+    // reference takes them of its angle rounded to float (and evaluates three
+    // trigonometric functions a view, 7 us of a 29 us call at 180 views)
+    const double norm = sqrt(norm2), c = ux / norm, s = uy / norm;
     const bool vertical = fabsf(p.src[0]) <= fabsf(p.src[1]);
     o.vertical = vertical ? 1 : 0;
     double detstep, slicestep, corr, p0;
