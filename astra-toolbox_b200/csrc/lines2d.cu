@@ -108,7 +108,8 @@ __device__ __forceinline__ int floor_texel(float q) { return __float_as_int(__fa
 
 constexpr int FP2D_GROUPS = LINES_WARPS / FP2D_PARTS;  // groups of 16 detectors x 4 views per CTA
 
-struct FP2DLinesLaunch {
+// CAP views' constants travel in the launch parameters.
+template <int CAP> struct FP2DLinesLaunch {
     // texel 0 of line 0 and byte pitch of a line: rows (rays that march over
     // rows, [0]) and columns ([1])
     const char *line0[2];
@@ -119,8 +120,8 @@ struct FP2DLinesLaunch {
     float out_scale;
     const float *res_b, *res_w;  // SIRT's residual in place of the projection: (b - A x) w
     union {
-        ParFPView par[FP2D_MAX_VIEWS];
-        b2t_view2d fan[FP2D_MAX_VIEWS];
+        ParFPView par[CAP];
+        b2t_view2d fan[CAP];
     };
 };
 
@@ -266,8 +267,8 @@ __device__ __forceinline__ void sum_part(const LineRay (&ray)[2], bool mixed, in
 // (1024^2 x 1440: 0.89, 0.97, 0.84 ms).  About ten instructions per sample at
 // half the issue rate: bound by the latency of the loads that miss L1 (one
 // load in eight).
-template <int KIND>
-__global__ void __launch_bounds__(LINES_THREADS) fp2d_lines_kernel(const __grid_constant__ FP2DLinesLaunch L)
+template <int KIND, int CAP>
+__global__ void __launch_bounds__(LINES_THREADS) fp2d_lines_kernel(const __grid_constant__ FP2DLinesLaunch<CAP> L)
 {
     __shared__ float red[FP2D_GROUPS][FP2D_PARTS][64];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -337,7 +338,7 @@ __global__ void __launch_bounds__(LINES_THREADS) fp2d_lines_kernel(const __grid_
 // backprojection
 // ---------------------------------------------------------------------------
 
-struct BP2DLinesLaunch {
+template <int CAP> struct BP2DLinesLaunch {
     const float *sino;  // row of the launch's first view
     long long sino_pitch;
     float *vol;
@@ -346,7 +347,7 @@ struct BP2DLinesLaunch {
     int win;  // pairs per staged row
     float out_scale;
     SirtUpdate2D upd;  // x set: SIRT's update in place of the backprojection
-    BPView2D views[BP2D_MAX_VIEWS];  // parallel: c[2] less 1/2
+    BPView2D views[CAP];  // parallel: c[2] less 1/2
 };
 
 // A staged view: its constants and the shared-memory byte address of its
@@ -417,8 +418,8 @@ __device__ __forceinline__ void bp_positions(const float *c, const uint64_t (&x2
 // buffers.  Bound by instruction issue (77 %) with the shared-memory data
 // pipe at 58 %: 1024^2 x 1440 takes 0.62 ms parallel and 0.94 ms fan; reading
 // bordered pairs of the sinogram through L1 instead took 0.84 and 1.56 ms.
-template <int KIND, int PX, int WS, int ROWS>
-__global__ void __launch_bounds__(LINES_THREADS) bp2d_lines_kernel(const __grid_constant__ BP2DLinesLaunch L)
+template <int KIND, int PX, int WS, int ROWS, int CAP>
+__global__ void __launch_bounds__(LINES_THREADS) bp2d_lines_kernel(const __grid_constant__ BP2DLinesLaunch<CAP> L)
 {
     constexpr int WY = LINES_WARPS / WS, NP = BP2D_PARTS / WS, NV = ROWS / WS;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -627,11 +628,11 @@ size_t lines_bytes(size_t lines, size_t n, size_t &total)
     return b;
 }
 
-template <int KIND>
-cudaError_t launch_fp(const FP2DLinesLaunch &L, cudaStream_t s)
+template <int KIND, int CAP>
+cudaError_t launch_fp(const FP2DLinesLaunch<CAP> &L, cudaStream_t s)
 {
     constexpr int D = 16 * FP2D_GROUPS;
-    fp2d_lines_kernel<KIND><<<dim3((L.nviews + 3) / 4, (L.ndet + D - 1) / D), LINES_THREADS, 0, s>>>(L);
+    fp2d_lines_kernel<KIND, CAP><<<dim3((L.nviews + 3) / 4, (L.ndet + D - 1) / D), LINES_THREADS, 0, s>>>(L);
     return cudaGetLastError();
 }
 
@@ -651,7 +652,8 @@ float bp_step(int kind, const BPView2D &C, const b2t_dims2d &d)
     return step;
 }
 
-template <int KIND, int PX, int WS, int ROWS> cudaError_t launch_bp_shape(BP2DLinesLaunch &L, float step, cudaStream_t s)
+template <int KIND, int PX, int WS, int ROWS, int CAP>
+cudaError_t launch_bp_shape(BP2DLinesLaunch<CAP> &L, float step, cudaStream_t s)
 {
     constexpr int TX = 8 * PX, WY = LINES_WARPS / WS, TY = 4 * WY;
     // the widest footprint of a tile, with a texel on both sides and one for
@@ -660,7 +662,7 @@ template <int KIND, int PX, int WS, int ROWS> cudaError_t launch_bp_shape(BP2DLi
     L.win = span < 160.0f ? ((int)span + 2) & ~1 : 160;
     const size_t smem = 2 * ROWS * (sizeof(BPRecord) + (size_t)L.win * sizeof(float2)) +
                         (WS > 1 ? (size_t)WY * BP2D_PARTS * 32 * PX * sizeof(float) : 0);
-    auto kern = bp2d_lines_kernel<KIND, PX, WS, ROWS>;
+    auto kern = bp2d_lines_kernel<KIND, PX, WS, ROWS, CAP>;
     if (smem > 47 * 1024) {  // (with the static part, 48 KB without asking)
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -675,8 +677,8 @@ template <int KIND, int PX, int WS, int ROWS> cudaError_t launch_bp_shape(BP2DLi
 // 25.2 / 19.2 / 13.0 / 9.5 us, at 512^2 x 720 109 / 119 / 158 / 227 us.
 constexpr long long LINES_BP_WARPS = 3600;
 
-template <int KIND>
-cudaError_t launch_bp(BP2DLinesLaunch &L, float step, cudaStream_t s)
+template <int KIND, int CAP>
+cudaError_t launch_bp(BP2DLinesLaunch<CAP> &L, float step, cudaStream_t s)
 {
     const long long tiles = (long long)((L.W + 31) / 32) * ((L.H + 3) / 4);
     if (8 * tiles <= LINES_BP_WARPS) return launch_bp_shape<KIND, 4, 8, 64>(L, step, s);
@@ -685,10 +687,13 @@ cudaError_t launch_bp(BP2DLinesLaunch &L, float step, cudaStream_t s)
     return launch_bp_shape<KIND, 4, 1, 32>(L, step, s);
 }
 
-}  // namespace
+// Views that a small launch's parameters hold (6 KB instead of 24 KB, which
+// the driver copies at every launch).
+constexpr int LINES_SMALL_VIEWS = 256;
 
-b2t_status fp2d_lines(const b2t_geom2d *g, uint32_t det_supersample, const float *vol, size_t vol_pitch, float *sino,
-                      size_t sino_pitch, int32_t mode, const float *res_b, const float *res_w, cudaStream_t s)
+template <int CAP>
+b2t_status fp_run(const b2t_geom2d *g, uint32_t det_supersample, const float *vol, size_t vol_pitch, float *sino,
+                  size_t sino_pitch, int32_t mode, const float *res_b, const float *res_w, cudaStream_t s)
 {
     const b2t_dims2d &d = g->dims;
     // which lines the rays march over: a parallel view's rays share the
@@ -704,8 +709,8 @@ b2t_status fp2d_lines(const b2t_geom2d *g, uint32_t det_supersample, const float
     if (cols) lines_bytes(d.vol_width, d.vol_height, total);
     Scratch sc;
     B2T_TRY(sc.alloc(total, s, "b2t_fp2d scratch (line copy)"));
-    const std::unique_ptr<FP2DLinesLaunch> keep(new FP2DLinesLaunch);
-    FP2DLinesLaunch &L = *keep;
+    const std::unique_ptr<FP2DLinesLaunch<CAP>> keep(new FP2DLinesLaunch<CAP>);
+    FP2DLinesLaunch<CAP> &L = *keep;
     L.res_b = res_b;
     L.res_w = res_w;
     L.pitch[0] = (d.vol_width + 2 * LINE_BORDER) * (uint32_t)sizeof(float2);
@@ -726,27 +731,28 @@ b2t_status fp2d_lines(const b2t_geom2d *g, uint32_t det_supersample, const float
     L.rays = det_supersample;
     L.accumulate = (mode == B2T_MODE_ADD) ? 1 : 0;
     L.out_scale = g->output_scale;
-    for (uint32_t c0 = 0; c0 < d.angles; c0 += FP2D_MAX_VIEWS) {
-        const uint32_t cn = std::min(d.angles - c0, (uint32_t)FP2D_MAX_VIEWS);
+    for (uint32_t c0 = 0; c0 < d.angles; c0 += CAP) {
+        const uint32_t cn = std::min(d.angles - c0, (uint32_t)CAP);
         L.a0 = (int)c0;
         L.nviews = (int)cn;
         for (uint32_t i = 0; i < cn; ++i) {
             if (g->kind == B2T_GEOM_PAR2D) par_fp_view(g->views[c0 + i], d, g->output_scale, L.par[i]);
             else L.fan[i] = g->views[c0 + i];
         }
-        const cudaError_t e = g->kind == B2T_GEOM_PAR2D ? launch_fp<B2T_GEOM_PAR2D>(L, s) : launch_fp<B2T_GEOM_FAN2D>(L, s);
+        const cudaError_t e = g->kind == B2T_GEOM_PAR2D ? launch_fp<B2T_GEOM_PAR2D, CAP>(L, s) : launch_fp<B2T_GEOM_FAN2D, CAP>(L, s);
         count_launches(1);
         B2T_CUDA_TRY(e, "fp2d launch");
     }
     return B2T_OK;
 }
 
-b2t_status bp2d_lines(const b2t_geom2d *g, int32_t fbp_weight, const float *sino, size_t sino_pitch, float *vol,
-                      size_t vol_pitch, int32_t mode, const SirtUpdate2D *update, cudaStream_t s)
+template <int CAP>
+b2t_status bp_run(const b2t_geom2d *g, int32_t fbp_weight, const float *sino, size_t sino_pitch, float *vol,
+                  size_t vol_pitch, int32_t mode, const SirtUpdate2D *update, cudaStream_t s)
 {
     const b2t_dims2d &d = g->dims;
-    const std::unique_ptr<BP2DLinesLaunch> keep(new BP2DLinesLaunch);
-    BP2DLinesLaunch &L = *keep;
+    const std::unique_ptr<BP2DLinesLaunch<CAP>> keep(new BP2DLinesLaunch<CAP>);
+    BP2DLinesLaunch<CAP> &L = *keep;
     L.upd = update ? *update : SirtUpdate2D{};
     L.sino_pitch = (long long)sino_pitch;
     L.vol = vol;
@@ -754,8 +760,8 @@ b2t_status bp2d_lines(const b2t_geom2d *g, int32_t fbp_weight, const float *sino
     L.W = d.vol_width; L.H = d.vol_height; L.ndet = d.dets;
     L.fbp = fbp_weight ? 1 : 0;
     L.out_scale = g->output_scale;
-    for (uint32_t c0 = 0; c0 < d.angles; c0 += BP2D_MAX_VIEWS) {
-        const uint32_t cn = std::min(d.angles - c0, (uint32_t)BP2D_MAX_VIEWS);
+    for (uint32_t c0 = 0; c0 < d.angles; c0 += CAP) {
+        const uint32_t cn = std::min(d.angles - c0, (uint32_t)CAP);
         L.sino = sino + (size_t)c0 * sino_pitch;
         L.nviews = (int)cn;
         float step = 0.0f;
@@ -766,11 +772,27 @@ b2t_status bp2d_lines(const b2t_geom2d *g, int32_t fbp_weight, const float *sino
             step = std::max(step, bp_step(g->kind, L.views[i], d));
         }
         const cudaError_t e =
-            g->kind == B2T_GEOM_PAR2D ? launch_bp<B2T_GEOM_PAR2D>(L, step, s) : launch_bp<B2T_GEOM_FAN2D>(L, step, s);
+            g->kind == B2T_GEOM_PAR2D ? launch_bp<B2T_GEOM_PAR2D, CAP>(L, step, s) : launch_bp<B2T_GEOM_FAN2D, CAP>(L, step, s);
         count_launches(1);
         B2T_CUDA_TRY(e, "bp2d launch");
     }
     return B2T_OK;
+}
+
+}  // namespace
+
+b2t_status fp2d_lines(const b2t_geom2d *g, uint32_t det_supersample, const float *vol, size_t vol_pitch, float *sino,
+                      size_t sino_pitch, int32_t mode, const float *res_b, const float *res_w, cudaStream_t s)
+{
+    auto run = g->dims.angles <= LINES_SMALL_VIEWS ? fp_run<LINES_SMALL_VIEWS> : fp_run<FP2D_MAX_VIEWS>;
+    return run(g, det_supersample, vol, vol_pitch, sino, sino_pitch, mode, res_b, res_w, s);
+}
+
+b2t_status bp2d_lines(const b2t_geom2d *g, int32_t fbp_weight, const float *sino, size_t sino_pitch, float *vol,
+                      size_t vol_pitch, int32_t mode, const SirtUpdate2D *update, cudaStream_t s)
+{
+    auto run = g->dims.angles <= LINES_SMALL_VIEWS ? bp_run<LINES_SMALL_VIEWS> : bp_run<BP2D_MAX_VIEWS>;
+    return run(g, fbp_weight, sino, sino_pitch, vol, vol_pitch, mode, update, s);
 }
 
 }  // namespace b2t
