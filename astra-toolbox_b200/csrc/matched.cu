@@ -382,6 +382,16 @@ b2t_status matched_bp3d_impl(const b2t_geom3d *g, const b2t_params3d *p, const v
         dirs[a] = dominant_axis(g->kind, g->views[a], d);
         need[dirs[a]] = true;
     }
+    // gathered per voxel where every view allows it (matched_gather.cu), else
+    // scattered; without memory for its weighted rows, scattered as well
+    const bool slab_asked =
+        (need[0] && matched_slab_eligible(g, p, 0, dirs)) || (need[1] && matched_slab_eligible(g, p, 1, dirs));
+    if (!slab_asked && !matched_force_plain() && matched_gather_eligible(g, p, dirs)) {
+        const b2t_status st = matched_gather(g, p, proj, proj_pitch, vol, vol_pitch, dtype,
+                                             (mode == B2T_MODE_ADD) ? 1 : 0, dirs, s);
+        if (st != B2T_ERR_NO_MEMORY) return st;
+        clear_error();
+    }
     const size_t px = d.vol_x + 4, py = d.vol_y + 4, pz = d.vol_z + 4;
     const size_t padded = px * py * pz;
     {

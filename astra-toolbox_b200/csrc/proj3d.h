@@ -205,6 +205,10 @@ b2t_status bp3d_impl(const b2t_geom3d *g, const b2t_params3d *p, const void *pro
 // use the pair layout (padded_elem_size).
 bool bp_pairs(int32_t dtype, const b2t_params3d *p);
 size_t padded_proj_bytes(const b2t_dims3d &d, int32_t dtype, bool pairs);
+// matched BP gathered per voxel: whether every view allows it, and the call
+bool matched_gather_eligible(const b2t_geom3d *g, const b2t_params3d *p, const std::vector<int> &dirs);
+b2t_status matched_gather(const b2t_geom3d *g, const b2t_params3d *p, const void *proj, size_t proj_pitch, void *vol,
+                          size_t vol_pitch, int32_t dtype, int accumulate, const std::vector<int> &dirs, cudaStream_t s);
 // The zero-padded projection buffer of projections proj (row pitch in
 // texels) in the layout bp_pairs selects.
 b2t_status pad_projections_impl(const void *proj, size_t pitch, const b2t_dims3d &d, void *padded, int32_t dtype,

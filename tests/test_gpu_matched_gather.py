@@ -1,0 +1,133 @@
+"""The exact adjoint gathered per voxel (B2T_MATCHED_PATH=gather: at any size) against the FP64 transpose and the
+scattered adjoint (B2T_MATCHED_PLAIN=1): volumes around the 8 x 8 x 64 and 16 x 16 x 64 tiles,
+detectors of every row spacing from 1/4 texel on, detector columns that
+run either way, off-centre and cropped detectors, split views, storage types,
+ADD mode, row pitches; views that the gather does not take are scattered."""
+import ctypes
+import importlib
+
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def _scatters():
+    out = (ctypes.c_uint64 * 4)()
+    assert importlib.import_module("astra-toolbox_b200._lib").load().b2t_matched_path_stats(out) == 0
+    return out[2] + out[3]
+
+
+def _vec(kind, n, pu, pv, flip=False, shift=(0.0, 0.0), so=150.0, od=60.0):
+    out = np.zeros((n, 12))
+    for i in range(n):
+        t = 2 * np.pi * i / n + 0.07
+        u, v = np.array([np.cos(t), np.sin(t), 0.0]), np.array([0.0, 0.0, 1.0])
+        ray = np.array([-np.sin(t), np.cos(t), 0.0])
+        c = ray * od + shift[0] * u + shift[1] * v
+        out[i] = np.concatenate([-ray * so if kind == 'cone_vec' else ray, c, pu * (-u if flip else u), pv * v])
+    return out
+
+
+def _check(astra, orc, pg, vg, monkeypatch, gathered=True, dtype="float32", keep=1.0):
+    pr = astra.Projector3D(pg, vg, {'ProjectionKernel': 'matched_bp'})
+    proj = np.random.default_rng(pr.vol_shape[0]).standard_normal(pr.proj_shape).astype(np.float32)
+    proj *= np.random.default_rng(1).random((1,) + pr.proj_shape[1:]) < keep
+    tp = torch.from_numpy(proj).cuda().to(getattr(torch, dtype))
+    monkeypatch.setenv("B2T_MATCHED_PATH", "gather")
+    _scatters()
+    a = torch.zeros(pr.vol_shape, device='cuda', dtype=tp.dtype)
+    pr.bp(tp, a)
+    n = _scatters()
+    assert gathered is None or (n == 0) == gathered
+    monkeypatch.setenv("B2T_MATCHED_PLAIN", "1")
+    b = torch.zeros_like(a)
+    pr.bp(tp, b)
+    monkeypatch.delenv("B2T_MATCHED_PLAIN")
+    assert _scatters() > 0
+    ref = orc.fp3d_transpose(pr.geom.kind, pr.geom.views_array(), tp.float().cpu().numpy(), pr.vol_shape,
+                             pr.geom.vol_scale)
+    # one rounding of the output in 16 bits, FP32 sums in another order else
+    tol = {"float32": 1e-5, "float16": 1e-3, "bfloat16": 8e-3}[dtype]
+    assert rel_l2(a.float().cpu().numpy(), ref) < tol
+    assert rel_l2(a.float().cpu().numpy(), b.float().cpu().numpy()) < tol
+    c = a.clone()
+    pr.bp(tp, c, mode=0)
+    assert rel_l2(c.float().cpu().numpy(), 2 * ref) < tol
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (63, 15, 17), (64, 16, 16), (65, 17, 15), (33, 50, 31), (130, 20, 40)])
+@pytest.mark.parametrize("kind", ["cone_vec", "parallel3d_vec"])
+def test_tile_edges(astra, orc, shape, kind, monkeypatch):
+    nz, ny, nx = shape
+    vg = astra.create_vol_geom(ny, nx, nz)
+    for n, flip in ((3, False), (17, True), (50, False)):
+        pg = astra.create_proj_geom(kind, 67, 75, _vec(kind, n, 1.0, 0.95, flip))
+        _check(astra, orc, pg, vg, monkeypatch)
+
+
+@pytest.mark.parametrize("pv", [0.45, 0.55, 0.75, 0.9, 1.2, 2.9])
+def test_row_spacings(astra, orc, pv, monkeypatch):
+    vg = astra.create_vol_geom(24, 30, 40)
+    for pu in (0.3, 1.0, 3.0):
+        for kind in ("cone_vec", "parallel3d_vec"):
+            pg = astra.create_proj_geom(kind, 41, 53, _vec(kind, 20, pu, pv, shift=(3.3, -2.7)))
+            # (edge columns of wide detectors have rows below a quarter of a texel
+            # apart at the finest; rows of more than 1 are scattered)
+            _check(astra, orc, pg, vg, monkeypatch, gathered=None if pv < 0.6 else pv * (150 / 210 if kind == "cone_vec" else 1) < 1.0)
+
+
+@pytest.mark.parametrize("keep", [0.0, 0.02, 0.3, 0.9])
+def test_zero_columns(astra, orc, keep, monkeypatch):
+    vg = astra.create_vol_geom(24, 40, 33)
+    for pu in (0.3, 1.0, 2.5):
+        pg = astra.create_proj_geom('cone_vec', 41, 70, _vec('cone_vec', 20, pu, 1.0))
+        _check(astra, orc, pg, vg, monkeypatch, keep=keep)
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+def test_storage(astra, orc, dtype, monkeypatch):
+    vg = astra.create_vol_geom(40, 36, 70, -20, 16, -22.0, 18.0, -30.0, 40.0)
+    pg = astra.create_proj_geom('cone', 1.1, 0.9, 60, 64, np.linspace(0, 2 * np.pi, 30, endpoint=False), 150.0, 60.0)
+    _check(astra, orc, pg, vg, monkeypatch, dtype=dtype)
+
+
+def test_anisotropic_voxels(astra, orc, monkeypatch):
+    vg = astra.create_vol_geom(40, 36, 30, -18, 18, -30.0, 30.0, -18.0, 18.0)
+    pg = astra.create_proj_geom('cone', 1.1, 0.9, 60, 64, np.linspace(0, 2 * np.pi, 30, endpoint=False), 150.0, 60.0)
+    _check(astra, orc, pg, vg, monkeypatch)
+
+
+@pytest.mark.parametrize("case", ["fine", "flipped_rows", "tilted"])
+def test_scattered_views(astra, orc, case, monkeypatch):
+    vg = astra.create_vol_geom(24, 30, 20)
+    v = _vec('cone_vec', 12, 1.0, 1.0)
+    if case == "fine":
+        v = _vec('cone_vec', 12, 1.0, 0.2)
+    elif case == "flipped_rows":
+        v[:, 9:12] *= -1
+    else:
+        v[3, 9] = 0.2
+    pg = astra.create_proj_geom('cone_vec', 40, 44, v)
+    _check(astra, orc, pg, vg, monkeypatch, gathered=False)
+
+
+def test_default_size(astra, orc):
+    """Above 3e8 voxel views the gather is the default, both blocks' shapes and
+    split views among them, and needs no scatter."""
+    for n, na in ((64, 1200), (128, 150)):
+        vg = astra.create_vol_geom(n, n, n)
+        pg = astra.create_proj_geom('cone', 1.0, 1.0, n, n, np.linspace(0, 2 * np.pi, na, endpoint=False), 4.0 * n, n)
+        pr = astra.Projector3D(pg, vg, {'ProjectionKernel': 'matched_bp'})
+        x = torch.randn(pr.vol_shape, device='cuda')
+        y = torch.rand(pr.proj_shape, device='cuda')
+        ax, aty = torch.zeros_like(y), torch.zeros_like(x)
+        pr.fp(x, ax)
+        _scatters()
+        pr.bp(y, aty)
+        assert _scatters() == 0
+        lhs, rhs = float((ax.double() * y.double()).sum()), float((x.double() * aty.double()).sum())
+        assert abs(lhs - rhs) < 1e-6 * float(ax.double().norm() * y.double().norm())
