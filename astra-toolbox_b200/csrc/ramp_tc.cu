@@ -371,8 +371,16 @@ bool ramp_tc_plan(uint32_t nu, long long M, RampTCPlan &plan)
     plan.M = M;
     plan.kh = (int)((nu + 1) / 2);
     plan.khp = (plan.kh + 15) & ~15;
-    const int t = (plan.kh + 127) / 128;
-    plan.bn = (((plan.kh + t - 1) / t) + 15) & ~15;
+    // tiles of up to 128 output columns; few rows (one sinogram) leave most SMs
+    // without a tile, and a tile's epilogue is a serial chain of 16-column
+    // chunks: narrower ones then, down to 32 columns, until half of the SMs
+    // have one.  The sums along K, and so the results, are the same.
+    // FBP of 720 rows of 768 columns: 18 tiles 157 us, 72 tiles 146.5 us.
+    const long long mtiles = (M + RT_BM - 1) / RT_BM;
+    for (int t = (plan.kh + 127) / 128;; ++t) {
+        plan.bn = (((plan.kh + t - 1) / t) + 15) & ~15;
+        if (plan.bn <= 32 || mtiles * t >= 74) break;
+    }
     plan.ntn = (plan.kh + plan.bn - 1) / plan.bn;
     plan.nhp = plan.ntn * plan.bn;
     plan.nkb = (plan.kh + RT_BK - 1) / RT_BK;
