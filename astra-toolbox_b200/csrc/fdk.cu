@@ -50,6 +50,10 @@ template <> __device__ __forceinline__ __nv_bfloat16 stf<__nv_bfloat16>(float v)
 
 constexpr int FILT_THREADS = 256;
 constexpr int FILT_OUT = 8;  // consecutive outputs per thread
+// Dynamic shared memory that a filter kernel may ask for.  Its limit is set to
+// this in every call, whatever the call needs: the limit belongs to the
+// kernel, and a call of another thread may set it before the launch.
+constexpr size_t FILT_SMEM = 200 * 1024;
 
 // Parker weight of view a at detector column offset fU (devFDK_ParkerWeight).
 __device__ __forceinline__ float parker_weight(float beta, float fU, const FDKWeights &P)
@@ -512,14 +516,14 @@ static b2t_status launch_filter(const void *src, size_t src_pitch, const b2t_dim
     const int nu = d.det_u;
     const size_t row_bytes = sizeof(float) * (3 * (size_t)nu + 32);
     const size_t tap_bytes = sizeof(float) * ((nu + 1) / 2 + 1);
-    const size_t budget = 200 * 1024;
+    const size_t budget = FILT_SMEM;
     if (row_bytes + tap_bytes > budget)
         return fail(B2T_ERR_UNSUPPORTED, "FDK filter: detector rows of %d pixels exceed shared memory", nu);
     int rows = (int)((budget - tap_bytes) / row_bytes);
     if (rows > 8) rows = 8;
     const size_t smem = rows * row_bytes + tap_bytes;
     auto kern = fdk_weight_filter_kernel<T>;
-    B2T_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    B2T_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FILT_SMEM),
                  "FDK filter smem attribute");
     const long long mtot = (long long)d.angles * d.det_v;
     const long long blocks = (mtot + rows - 1) / rows;
@@ -555,14 +559,14 @@ static b2t_status launch_toeplitz(const void *src, size_t src_pitch, const b2t_d
 {
     const int nu = d.det_u;
     const size_t row_bytes = sizeof(float) * (3 * (size_t)nu + 32);
-    const size_t budget = 200 * 1024;
+    const size_t budget = FILT_SMEM;
     if (row_bytes > budget)
         return fail(B2T_ERR_UNSUPPORTED, "filter: detector rows of %d pixels exceed shared memory", nu);
     int rows = (int)(budget / row_bytes);
     if (rows > 8) rows = 8;
     const size_t smem = rows * row_bytes;
     auto kern = fdk_weight_toeplitz_kernel<T>;
-    B2T_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    B2T_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FILT_SMEM),
                  "filter smem attribute");
     const long long mtot = (long long)d.angles * d.det_v;
     const long long blocks = (mtot + rows - 1) / rows;
@@ -581,7 +585,7 @@ static b2t_status launch_split(const void *src, size_t src_pitch, const b2t_dims
                                long long dst_row, long long dst_v, int blocks, size_t smem, cudaStream_t s)
 {
     auto kern = fdk_split_kernel<T>;
-    B2T_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    B2T_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FILT_SMEM),
                  "ramp filter split smem attribute");
     kern<<<blocks, SPLIT_THREADS, smem, s>>>(static_cast<const T *>(src), (long long)src_pitch, (int)d.det_u,
                                              (int)d.angles, (int)d.det_v, P, rel_dev, a, khp, M,
@@ -637,7 +641,7 @@ static b2t_status run_filter(const b2t_dims3d &d, const FDKWeights &P, const std
             const long long blocks = (M + SPLIT_ROWS - 1) / SPLIT_ROWS;
             const size_t wrow = (size_t)d.det_u + 2 * RAMP_TC_BAND + 12;  // PADL + nu + PADR
             const size_t smem = sizeof(float) * SPLIT_ROWS * (wrow + wrow / 8 + 1);
-            if (blocks > 0x7fffffffLL || smem > 200 * 1024)
+            if (blocks > 0x7fffffffLL || smem > FILT_SMEM)
                 return fail(B2T_ERR_UNSUPPORTED, "ramp filter: %lld rows of %u columns are too many", M, d.det_u);
             if (dtype == B2T_F32)
                 st = launch_split<float>(src, src_pitch, d, P, rel_dev, a, plan.khp, M, dst, dst_row, dst_v,

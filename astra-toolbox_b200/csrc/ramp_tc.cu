@@ -71,6 +71,7 @@ constexpr uint32_t RT_TMEM_COLS = 512;
 constexpr int RT_A_TILE = RT_BM * RT_BK * 2;         // bytes of one A term tile
 constexpr int RT_EPI_STRIDE = 33;                    // floats per staged row (conflict-free)
 constexpr int RT_EPI_BYTES = 4 * 32 * RT_EPI_STRIDE * 4;
+constexpr int RT_MAX_BN = 128;                       // output columns of the widest tile
 constexpr long long RT_WAIT = 2000000000LL;          // clock cycles, about a second
 
 struct RampTCLaunch {
@@ -377,7 +378,7 @@ bool ramp_tc_plan(uint32_t nu, long long M, RampTCPlan &plan)
     // have one.  The sums along K, and so the results, are the same.
     // FBP of 720 rows of 768 columns: 18 tiles 157 us, 72 tiles 146.5 us.
     const long long mtiles = (M + RT_BM - 1) / RT_BM;
-    for (int t = (plan.kh + 127) / 128;; ++t) {
+    for (int t = (plan.kh + RT_MAX_BN - 1) / RT_MAX_BN;; ++t) {
         plan.bn = (((plan.kh + t - 1) / t) + 15) & ~15;
         if (plan.bn <= 32 || mtiles * t >= 74) break;
     }
@@ -389,13 +390,19 @@ bool ramp_tc_plan(uint32_t nu, long long M, RampTCPlan &plan)
     return true;
 }
 
+// Bytes of one stage, and of a CTA's shared memory, for tiles of bn columns.
+constexpr int rt_stage_bytes(int bn) { return 3 * RT_A_TILE + 3 * bn * RT_BK * 2; }
+constexpr int rt_smem(int bn) { return 1024 + RT_STAGES * rt_stage_bytes(bn) + RT_EPI_BYTES + 8 * (2 * RT_STAGES + 5) + 16; }
+
 template <typename T>
-static b2t_status launch_ramp(const RampTCLaunch &L, int grid, size_t smem, cudaStream_t s)
+static b2t_status launch_ramp(const RampTCLaunch &L, int grid, cudaStream_t s)
 {
     auto kern = ramp_tc_kernel<T>;
-    B2T_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    // the widest tile's in every call: the limit belongs to the kernel, and a
+    // call of another thread may set it between here and the launch
+    B2T_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, rt_smem(RT_MAX_BN)),
                  "ramp filter smem attribute");
-    kern<<<grid, RT_THREADS, smem, s>>>(L);
+    kern<<<grid, RT_THREADS, rt_smem(L.bn), s>>>(L);
     count_launches(1);
     B2T_CUDA_TRY(cudaGetLastError(), "ramp filter launch");
     return B2T_OK;
@@ -450,9 +457,8 @@ b2t_status ramp_tc_filter(const RampTCPlan &P, const __nv_bfloat16 *a, __nv_bflo
     L.ntn = P.ntn;
     const long long mtiles = (P.M + RT_BM - 1) / RT_BM;
     L.ntiles = mtiles * P.ntn;
-    L.stage_bytes = 3 * RT_A_TILE + 3 * P.bn * RT_BK * 2;
+    L.stage_bytes = rt_stage_bytes(P.bn);
     L.idesc = umma_idesc_bf16_f32(RT_BM, (uint32_t)P.bn);
-    const size_t smem = 1024 + (size_t)RT_STAGES * L.stage_bytes + RT_EPI_BYTES + 8 * (2 * RT_STAGES + 5) + 16;
     int dev = 0, sms = 0;
     b2t_status st = B2T_OK;
     cudaError_t e = cudaGetDevice(&dev);
@@ -460,9 +466,9 @@ b2t_status ramp_tc_filter(const RampTCPlan &P, const __nv_bfloat16 *a, __nv_bflo
     if (e != cudaSuccess) st = cuda_fail(e, "ramp filter device query");
     if (st == B2T_OK) {
         const int grid = (int)std::min<long long>(L.ntiles, (long long)sms);
-        if (dtype == B2T_F32) st = launch_ramp<float>(L, grid, smem, s);
-        else if (dtype == B2T_F16) st = launch_ramp<__half>(L, grid, smem, s);
-        else st = launch_ramp<__nv_bfloat16>(L, grid, smem, s);
+        if (dtype == B2T_F32) st = launch_ramp<float>(L, grid, s);
+        else if (dtype == B2T_F16) st = launch_ramp<__half>(L, grid, s);
+        else st = launch_ramp<__nv_bfloat16>(L, grid, s);
     }
     delete Lp;
     return st;
