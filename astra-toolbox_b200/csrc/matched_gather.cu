@@ -42,6 +42,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstdlib>
 #include <string>
@@ -82,6 +83,7 @@ struct MGPrep {
     MGColumn *cols;     // [view][u]
     MGRecord *recs;     // [view]
     int *live;          // [view][u]: 1 where the column holds a value other than zero (cleared before)
+    int *bad;           // [view]: 1 where some weighted value is infinite or NaN (cleared before)
     int nu, nv, na, pitch, half;
     int nviews, first;  // views of this launch, index of its first one in the gather's order
     float f1[2], f2[2], mul[2];
@@ -94,7 +96,7 @@ struct MGLaunch {
     const float *rows;
     const MGColumn *cols;
     const MGRecord *recs;
-    const int *live;
+    const int *live, *bad;
     int nu, nv, pitch, half;
     int nx, ny, nz;
     int nx_views, nviews;  // x-major views come first
@@ -140,9 +142,11 @@ template <typename T> __global__ void __launch_bounds__(256) matched_prep_kernel
         const int v = v0 + threadIdx.x;
         const float y = tile[threadIdx.x][r];
         const bool any = __any_sync(0xffffffffu, y != 0.0f);
+        const bool off = __any_sync(0xffffffffu, !(fabsf(y) <= FLT_MAX));
         if (u0 + r >= L.nu) continue;
         if (v < L.pitch) L.rows[(gi * L.nu + u0 + r) * L.pitch + v] = y;
         if (any && threadIdx.x == 0) L.live[gi * L.nu + u0 + r] = 1;
+        if (off && threadIdx.x == 0) L.bad[gi] = 1;
     }
     if (blockIdx.y == 0 && threadIdx.y == 0 && u < L.nu) {
         // rows are counted from `half`, near the detector's centre
@@ -204,8 +208,11 @@ struct MGWalk {
     int *texels;        // and their base texels k1
 };
 
-// NT: terms of c_u(z), at least 2 / Q for every column of the walk.
-template <int T, int NT> __device__ __forceinline__ void mg_walk(const MGWalk &W, int lane)
+// NT: terms of c_u(z), at least 2 / Q for every column of the walk.  The NT rows
+// read may lie outside the support of hat, where its zero takes them out;
+// GUARD: some value of the view is infinite or NaN, and those rows are left
+// out by a comparison.
+template <int T, int NT, bool GUARD> __device__ __forceinline__ void mg_walk(const MGWalk &W, int lane)
 {
     const uint64_t M2 = pk2(MG_M, MG_M), nM2 = pk2(-MG_M, -MG_M), one2 = pk2(1.0f, 1.0f);
     const float tlo = MG_M + W.vlo, thi = MG_M + W.vhi;
@@ -271,8 +278,13 @@ template <int T, int NT> __device__ __forceinline__ void mg_walk(const MGWalk &W
 #pragma unroll
             for (int k = 0; k < NT; ++k) {
                 const float2 df = upk2(d);
-                const uint64_t h = pk2(__saturatef(1.0f - fabsf(df.x)), __saturatef(1.0f - fabsf(df.y)));
-                const uint64_t y = pk2(__ldg(pa + k), __ldg(pb + k));
+                const float ha = __saturatef(1.0f - fabsf(df.x)), hb = __saturatef(1.0f - fabsf(df.y));
+                float ya = __ldg(pa + k), yb = __ldg(pb + k);
+                if (GUARD) {
+                    ya = ha > 0.0f ? ya : 0.0f;
+                    yb = hb > 0.0f ? yb : 0.0f;
+                }
+                const uint64_t h = pk2(ha, hb), y = pk2(ya, yb);
                 c = k == 0 ? mul2(h, y) : fma2(h, y, c);
                 if (k + 1 < NT) d = add2(d, Q2);
             }
@@ -353,10 +365,11 @@ __global__ void __launch_bounds__(32 * T, 1024 / (32 * T)) matched_gather_kernel
                 W.rows = L.rows + (long long)i * L.nu * L.pitch;
                 const float dmax = fmaxf(fmaf((float)ua - uc, ra.y, ra.x), fmaf((float)ub - uc, ra.y, ra.x));
                 const float terms = 2.0f * dmax / fmaf(rb.z, sf, rb.w) * 1.00001f;
-                if (terms <= 2.0f) mg_walk<T, 2>(W, lane);
-                else if (terms <= 3.0f) mg_walk<T, 3>(W, lane);
-                else if (terms <= 4.0f) mg_walk<T, 4>(W, lane);
-                else mg_walk<T, MG_PAD>(W, lane);
+                if (__ldg(L.bad + i)) mg_walk<T, MG_PAD, true>(W, lane);
+                else if (terms <= 2.0f) mg_walk<T, 2, false>(W, lane);
+                else if (terms <= 3.0f) mg_walk<T, 3, false>(W, lane);
+                else if (terms <= 4.0f) mg_walk<T, 4, false>(W, lane);
+                else mg_walk<T, MG_PAD, false>(W, lane);
             }
         }
         __syncthreads();  // the other direction's warps take other rows of the tile
@@ -518,14 +531,16 @@ b2t_status matched_gather(const b2t_geom3d *g, const b2t_params3d *p, const void
     B2T_TRY(rows.alloc(ncol * L.pitch * sizeof(float), s, "matched bp weighted rows"));
     B2T_TRY(cols.alloc(ncol * sizeof(MGColumn), s, "matched bp columns"));
     B2T_TRY(recs.alloc(d.angles * sizeof(MGRecord), s, "matched bp views"));
-    B2T_TRY(live.alloc(ncol * sizeof(int), s, "matched bp live columns"));
-    B2T_CUDA_TRY(cudaMemsetAsync(live.as<void>(), 0, ncol * sizeof(int), s), "matched bp live columns");
+    const size_t flags = (ncol + d.angles) * sizeof(int);  // live, then bad
+    B2T_TRY(live.alloc(flags, s, "matched bp live columns"));
+    B2T_CUDA_TRY(cudaMemsetAsync(live.as<void>(), 0, flags, s), "matched bp live columns");
     const size_t vox = (size_t)d.vol_x * d.vol_y * d.vol_z;
     if (L.splits > 1) B2T_TRY(part.alloc(L.splits * vox * sizeof(float), s, "matched bp partial volumes"));
     L.rows = rows.as<float>();
     L.cols = cols.as<MGColumn>();
     L.recs = recs.as<MGRecord>();
     L.live = live.as<int>();
+    L.bad = L.live + ncol;
     {
         auto *Pp = new MGPrep;
         MGPrep &P = *Pp;
@@ -535,6 +550,7 @@ b2t_status matched_gather(const b2t_geom3d *g, const b2t_params3d *p, const void
         P.cols = cols.as<MGColumn>();
         P.recs = recs.as<MGRecord>();
         P.live = live.as<int>();
+        P.bad = P.live + ncol;
         P.nu = L.nu;
         P.nv = L.nv;
         P.na = (int)d.angles;

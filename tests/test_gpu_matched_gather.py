@@ -131,3 +131,39 @@ def test_default_size(astra, orc):
         assert _scatters() == 0
         lhs, rhs = float((ax.double() * y.double()).sum()), float((x.double() * aty.double()).sum())
         assert abs(lhs - rhs) < 1e-6 * float(ax.double().norm() * y.double().norm())
+
+
+@pytest.mark.parametrize("value", [float('nan'), float('inf'), -float('inf')])
+@pytest.mark.parametrize("dtype", ["float32", "float16"])
+@pytest.mark.parametrize("pv", [0.45, 0.95, 1.3])
+def test_non_finite_values(astra, orc, pv, dtype, value, monkeypatch):
+    """A dead pixel reaches the voxels that its ray meets and no others: in
+    the detector's first and last rows (rows past them are read with the
+    weight zero, for voxels below and above the detector's coverage) and inside
+    it.  (Weights below 1e-4 of a ray's largest one may round to nothing.)"""
+    vg = astra.create_vol_geom(24, 30, 70)
+    pg = astra.create_proj_geom('cone_vec', 41, 53, _vec('cone_vec', 9, 1.0, pv, shift=(1.3, -0.7)))
+    pr = astra.Projector3D(pg, vg, {'ProjectionKernel': 'matched_bp'})
+    rng = np.random.default_rng(4)
+    proj = rng.standard_normal(pr.proj_shape).astype(np.float32)
+    dead = np.zeros(pr.proj_shape, dtype=np.float32)
+    for pos in ((0, 2, 25), (40, 2, 31), (17, 5, 20), (0, 7, 3)):
+        dead[pos] = 1.0
+    back = lambda p: orc.fp3d_transpose(pr.geom.kind, pr.geom.views_array(), p, pr.vol_shape, pr.geom.vol_scale)
+    weight = back(dead)
+    met, missed = weight > 1e-4 * weight.max(), weight == 0
+    assert met.any() and missed.any()
+    tp = torch.from_numpy(np.where(dead > 0, np.float32(value), proj)).cuda().to(getattr(torch, dtype))
+    finite = np.where(dead > 0, 0.0, tp.float().cpu().numpy()).astype(np.float32)
+    ref = back(finite)
+    for path, name in (("B2T_MATCHED_PATH", "gather"), ("B2T_MATCHED_PLAIN", "1")):
+        monkeypatch.setenv(path, name)
+        _scatters()
+        out = torch.zeros(pr.vol_shape, device='cuda', dtype=tp.dtype)
+        pr.bp(tp, out)
+        monkeypatch.delenv(path)
+        assert (_scatters() == 0) == (name == "gather")
+        got = out.float().cpu().numpy()
+        assert not np.isfinite(got[met]).any(), path
+        assert np.isfinite(got[missed]).all(), path
+        assert rel_l2(got[missed], ref[missed]) < {"float32": 1e-5, "float16": 1e-3}[dtype]
