@@ -43,6 +43,7 @@ constexpr uint32_t SPLIT_BITS = 0x4B400000u;  // bits of SPLIT_M
 constexpr int LINE_BORDER = 2;                // zero texels on both sides of a line
 constexpr int LINES_THREADS = 256;
 constexpr int LINES_WARPS = LINES_THREADS / 32;
+constexpr int LINES_MAX_WIN = 160;            // pairs of a staged sinogram row (bp2d_lines), even
 
 // Pairs of line l at out[l * pitch + k + 2], k in [-2, n + 2).
 struct LineSet {
@@ -657,16 +658,20 @@ cudaError_t launch_bp_shape(BP2DLinesLaunch<CAP> &L, float step, cudaStream_t s)
 {
     constexpr int TX = 8 * PX, WY = LINES_WARPS / WS, TY = 4 * WY;
     // the widest footprint of a tile, with a texel on both sides and one for
-    // rounding, up to 160 pairs (wider ones are read from the sinogram)
+    // rounding, up to LINES_MAX_WIN pairs (wider ones are read from the sinogram)
     const float span = step * (float)(std::max(TX, TY)) + 4.0f;
-    L.win = span < 160.0f ? ((int)span + 2) & ~1 : 160;
-    const size_t smem = 2 * ROWS * (sizeof(BPRecord) + (size_t)L.win * sizeof(float2)) +
-                        (WS > 1 ? (size_t)WY * BP2D_PARTS * 32 * PX * sizeof(float) : 0);
+    L.win = span < (float)LINES_MAX_WIN ? ((int)span + 2) & ~1 : LINES_MAX_WIN;
+    auto bytes = [](int win) {
+        return 2 * ROWS * (sizeof(BPRecord) + (size_t)win * sizeof(float2)) +
+               (WS > 1 ? (size_t)WY * BP2D_PARTS * 32 * PX * sizeof(float) : 0);
+    };
+    const size_t smem = bytes(L.win);
     auto kern = bp2d_lines_kernel<KIND, PX, WS, ROWS, CAP>;
-    if (smem > 47 * 1024) {  // (with the static part, 48 KB without asking)
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    // the kernel's own maximum in every call: the limit belongs to the kernel,
+    // and a call of another thread may set it between here and the launch
+    const cudaError_t e =
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(LINES_MAX_WIN));
+    if (e != cudaSuccess) return e;
     kern<<<dim3((L.W + TX - 1) / TX, (L.H + TY - 1) / TY), LINES_THREADS, smem, s>>>(L);
     return cudaGetLastError();
 }

@@ -42,6 +42,22 @@ def _check(calls, n):
         assert torch.equal(got, ref)
 
 
+@pytest.mark.parametrize("n,views", [(64, 5000), (240, 3000), (480, 2000), (600, 2000)])
+def test_backprojections_of_different_windows(astra, n, views):
+    """Detectors of one pixel and of half a pixel: the same kernel, with
+    windows of staged sinogram rows of different widths (sizes of every split
+    of the views over warps; several launches a call, so that the threads are
+    mostly inside the library)."""
+    def call(px):
+        ang = np.linspace(0, np.pi, views, endpoint=False)
+        pr = astra.Projector2D(astra.create_proj_geom('parallel', px, int(1.5 * n / px), ang),
+                               astra.create_vol_geom(n, n))
+        sino, vol = torch.rand(pr.proj_shape, device='cuda'), torch.zeros(pr.vol_shape, device='cuda')
+        return lambda: pr.bp(sino, vol)
+
+    _check([call(1.0), call(0.5)], 1000 if n < 400 else 300)
+
+
 @pytest.mark.parametrize("filter_type", ["ram-lak", "hann"])
 def test_filters_of_different_rows(astra, filter_type):
     """Few and many rows, short and long: tensor-core tiles of different
