@@ -171,8 +171,8 @@ __device__ __forceinline__ void sum_part(const LineRay (&ray)[2], bool mixed, in
     int ulo = INT_MAX, uhi = INT_MIN, ilo = INT_MIN, ihi = INT_MAX;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-        lo[j] = max(ray[j].lo, part_begin(p, ray[j].n0, FP2D_PARTS));
-        hi[j] = min(ray[j].hi, part_begin(p + 1, ray[j].n0, FP2D_PARTS) - 1);
+        lo[j] = max(ray[j].lo, slice_begin(p, ray[j].n0));
+        hi[j] = min(ray[j].hi, slice_begin(p + 1, ray[j].n0) - 1);
         if (ray[j].lo <= ray[j].hi) {
             const bool some = lo[j] <= hi[j];
             ulo = min(ulo, some ? lo[j] : INT_MAX);
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(LINES_THREADS) fp2d_lines_kernel(const __grid_
             const int det = min(det0 + 8 * j, L.ndet - 1);
             Ray2D q;
             if constexpr (KIND == B2T_GEOM_PAR2D) q = par_ray2d(L.par[vi], det, r, R);
-            else q = fan_ray2d(L.fan[vi], L.W, L.H, det, r, R, L.out_scale);
+            else q = fan_ray2d(L.fan[vi], fan_horizontal(L.fan[vi], det), L.W, L.H, det, r, R, L.out_scale);
             const int o = q.horizontal ? 1 : 0;
             ray[j].A = q.A;
             ray[j].B = q.B;

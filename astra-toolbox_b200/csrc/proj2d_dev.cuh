@@ -55,6 +55,13 @@ __host__ __device__ __forceinline__ int part_begin(int p, int n, int parts)
     return (int)((long long)n * p / parts);
 }
 
+// Parts of a ray's slices begin at multiples of four (the direct bodies sum
+// four slices at a time and test once for the end of a part).
+__host__ __device__ __forceinline__ int slice_begin(int p, int n)
+{
+    return p < FP2D_PARTS ? part_begin(p, n, FP2D_PARTS) & ~3 : n;
+}
+
 // A ray: sample position q(slice) = A slice + B in texels (texel i at q = i)
 // of the line along the other axis; horizontal: slices are columns.
 struct Ray2D {
@@ -73,19 +80,26 @@ __device__ __forceinline__ Ray2D par_ray2d(const ParFPView &V, int det, int r, i
     return q;
 }
 
-// Sub-ray r of R of detector det of a fan view, scaled for the mean over R.
-__device__ __forceinline__ Ray2D fan_ray2d(const b2t_view2d &V, int W, int H, int det, int r, int R, float out_scale)
+// Whether a fan view's rays to detector det march over columns: the choice of
+// every ray, in float as the reference evaluates it.
+__device__ __forceinline__ bool fan_horizontal(const b2t_view2d &V, int det)
 {
-    Ray2D q;
-    // per-ray orientation choice, in float as the reference evaluates it
     const float fdx = fabsf(fmaf((float)det, V.det_u[0], V.det_s[0]) + 0.5f - V.src[0]);
     const float fdy = fabsf(fmaf((float)det, V.det_u[1], V.det_s[1]) + 0.5f - V.src[1]);
-    q.horizontal = !(fdy > fdx);
+    return !(fdy > fdx);
+}
+
+// Sub-ray r of R of detector det of a fan view, scaled for the mean over R.
+__device__ __forceinline__ Ray2D fan_ray2d(const b2t_view2d &V, bool horizontal, int W, int H, int det, int r, int R,
+                                           float out_scale)
+{
+    Ray2D q;
+    q.horizontal = horizontal;
     // ray set-up in FP64: the source sits far from the origin
     const double fdet = det + (0.5 + r) / (double)R;
     const double DX = V.det_s[0] + fdet * V.det_u[0];
     const double DY = V.det_s[1] + fdet * V.det_u[1];
-    if (q.horizontal) {
+    if (horizontal) {
         const double alpha = (V.src[1] - DY) / (V.src[0] - DX);
         const double beta = V.src[1] - alpha * V.src[0];
         q.corr = (float)(sqrt(alpha * alpha + 1.0) * out_scale / R);
@@ -102,22 +116,76 @@ __device__ __forceinline__ Ray2D fan_ray2d(const b2t_view2d &V, int W, int H, in
 }
 
 // Sum of the samples of a ray over slices s0, s0 + ds, ...; with ds = 1 from
-// slice 0 all of them, in FP2D_PARTS partial sums.
-__device__ __forceinline__ float sum_ray2d(const float *vol, long long pitch, int W, int H, const Ray2D &q, int s0,
-                                           int ds)
+// slice 0 all of them, in FP2D_PARTS partial sums.  COLS: the slices are
+// columns.
+//
+// Bound by the latency of the loads; the compiler unrolls one plain loop with
+// four samples' loads in flight, and a loop within a loop costs it (one view of
+// a 4096^2 image over rows: 283 us; a loop for every part 373 us; the choice of
+// direction inside the loop over sub-rays, or that loop around a single
+// ray, 300 to 470 us; run-time strides took the batched projections 1.15 to 1.18
+// times as long).  Hence the three tests in place of four loops, and the
+// branches on direction and on one sub-ray around everything else.
+template <bool COLS>
+__device__ __forceinline__ float sum_slices2d(const float *vol, long long pitch, int W, int H, const Ray2D &q, int s0,
+                                              int ds)
 {
-    const int n0 = q.horizontal ? W : H, n = q.horizontal ? H : W;
-    const long long st0 = q.horizontal ? 1 : pitch, st = q.horizontal ? pitch : 1;
-    float tot = 0.0f;
-    const int parts = ds == 1 ? FP2D_PARTS : 1;
-    for (int p = 0; p < parts; ++p) {
-        const int end = part_begin(p + 1, n0, parts);
-        float sum = 0.0f;
-        for (int sl = part_begin(p, n0, parts) + s0; sl < end; sl += ds)
-            sum += lerp_line(vol + sl * st0, st, n, fmaf((float)sl, q.A, q.B));
-        tot += sum;
+    const int n0 = COLS ? W : H;
+    auto sample = [&](int sl) {
+        const float x = fmaf((float)sl, q.A, q.B);
+        return COLS ? lerp_line(vol + sl, pitch, H, x) : lerp_line(vol + (long long)sl * pitch, 1, W, x);
+    };
+    float tot = 0.0f, sum = 0.0f;
+    if (ds != 1) {
+        for (int sl = s0; sl < n0; sl += ds) sum += sample(sl);
+        return sum;
     }
-    return tot;
+    static_assert(FP2D_PARTS == 4, "three ends between parts");
+    const int e1 = slice_begin(1, n0), e2 = slice_begin(2, n0), e3 = slice_begin(3, n0);
+    auto fold = [&](int sl) {
+        if (sl == e1 || sl == e2 || sl == e3) {
+            tot += sum;
+            sum = 0.0f;
+        }
+    };
+    int sl = 0;
+#pragma unroll 1
+    for (; sl + 3 < n0; sl += 4) {
+        float v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = sample(sl + i);
+        fold(sl);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum += v[i];
+    }
+    fold(sl);
+    for (; sl < n0; ++sl) sum += sample(sl);
+    return tot + sum;
+}
+
+// Sum over the R sub-rays of detector det: of a parallel view unscaled (all
+// share V.corr), of a fan view scaled.
+template <bool COLS>
+__device__ __forceinline__ float par_rays2d(const float *vol, long long pitch, int W, int H, const ParFPView &V, int det,
+                                            int R, int s0, int ds)
+{
+    if (R == 1) return sum_slices2d<COLS>(vol, pitch, W, H, par_ray2d(V, det, 0, 1), s0, ds);
+    float acc = 0.0f;
+    for (int r = 0; r < R; ++r) acc += sum_slices2d<COLS>(vol, pitch, W, H, par_ray2d(V, det, r, R), s0, ds);
+    return acc;
+}
+template <bool COLS>
+__device__ __forceinline__ float fan_rays2d(const float *vol, long long pitch, int W, int H, const b2t_view2d &V, int det,
+                                            int R, float out_scale, int s0, int ds)
+{
+    auto ray = [&](int r, int n, float acc) {
+        const Ray2D q = fan_ray2d(V, COLS, W, H, det, r, n, out_scale);
+        return fmaf(sum_slices2d<COLS>(vol, pitch, W, H, q, s0, ds), q.corr, acc);
+    };
+    if (R == 1) return ray(0, 1, 0.0f);
+    float acc = 0.0f;
+    for (int r = 0; r < R; ++r) acc = ray(r, R, acc);
+    return acc;
 }
 
 // Parallel-beam line integral of detector `det` (R sub-rays), scaled; over
@@ -125,8 +193,8 @@ __device__ __forceinline__ float sum_ray2d(const float *vol, long long pitch, in
 __device__ __forceinline__ float fp2d_par_ray(const float *vol, long long pitch, int W, int H, const ParFPView &V,
                                               int det, int R, int s0 = 0, int ds = 1)
 {
-    float acc = 0.0f;
-    for (int r = 0; r < R; ++r) acc += sum_ray2d(vol, pitch, W, H, par_ray2d(V, det, r, R), s0, ds);
+    const float acc = V.vertical ? par_rays2d<false>(vol, pitch, W, H, V, det, R, s0, ds)
+                                 : par_rays2d<true>(vol, pitch, W, H, V, det, R, s0, ds);
     return __fmul_rn(acc, V.corr / (float)R);  // (not fused into an accumulating caller)
 }
 
@@ -135,56 +203,72 @@ __device__ __forceinline__ float fp2d_par_ray(const float *vol, long long pitch,
 __device__ __forceinline__ float fp2d_fan_ray(const float *vol, long long pitch, int W, int H, const b2t_view2d &V,
                                               int det, int R, float out_scale, int s0 = 0, int ds = 1)
 {
-    float acc = 0.0f;
-    for (int r = 0; r < R; ++r) {
-        const Ray2D q = fan_ray2d(V, W, H, det, r, R, out_scale);
-        acc = fmaf(sum_ray2d(vol, pitch, W, H, q, s0, ds), q.corr, acc);
-    }
-    return acc;
+    return fan_horizontal(V, det) ? fan_rays2d<true>(vol, pitch, W, H, V, det, R, out_scale, s0, ds)
+                                  : fan_rays2d<false>(vol, pitch, W, H, V, det, R, out_scale, s0, ds);
 }
 
 // Backprojection sum of pixel (X, Y) over views [0, nviews) of `views`
 // (sinogram rows row0 .. row0 + nviews - 1), R x R sub-pixels, unscaled, in
-// BP2D_PARTS partial sums.
+// BP2D_PARTS partial sums.  ONE: R is 1 (the short ranges of a batch's small
+// problems show the loops over sub-pixels).
+template <bool ONE>
+__device__ __forceinline__ float bp2d_pixel_sum(const float *sino, long long sino_pitch, int row0, int nviews,
+                                                const BPView2D *views, int W, int H, int ndet, int R, int kind, int fbp,
+                                                int X, int Y)
+{
+    const float sub = 1.0f / (float)R;
+    auto add_view = [&](int i, float &acc) {
+        const BPView2D &C = views[i];
+        const float *row = sino + (long long)(row0 + i) * sino_pitch;
+        for (int ix = 0; ix < (ONE ? 1 : R); ++ix) {
+            for (int iy = 0; iy < (ONE ? 1 : R); ++iy) {
+                float x = (float)X - 0.5f * (float)W + 0.5f;
+                float y = (float)Y - 0.5f * (float)H + 0.5f;
+                if (!ONE && R > 1) {
+                    x += -0.5f + 0.5f * sub + (float)ix * sub;
+                    y += -0.5f + 0.5f * sub + (float)iy * sub;
+                }
+                if (kind == B2T_GEOM_PAR2D) {
+                    // T - 1/2, T = x c - y s + offset (par_bp.cu:78-81)
+                    const float q = fmaf(x, C.c[0], fmaf(-y, C.c[1], C.c[2] - 0.5f));
+                    acc = fmaf(lerp_line(row, 1, ndet, q), C.c[3], acc);
+                } else {
+                    // world y is flipped (fan_bp.cu:73)
+                    const float yw = -y;
+                    const float num = fmaf(x, C.c[1], fmaf(yw, C.c[2], C.c[0]));
+                    const float den = fmaf(x, C.c[4], fmaf(yw, C.c[5], C.c[3]));
+                    const float fr = rcp_newton(den);
+                    const float w = fbp ? fr * fr : fr;
+                    acc = fmaf(lerp_line(row, 1, ndet, fmaf(num, fr, -0.5f)), w, acc);
+                }
+            }
+        }
+    };
+    float tot = 0.0f;
+    if (nviews <= BP2D_PARTS) {
+        // a view or none in every part (4096^2, one view: 180 us with the loop below)
+        for (int i = 0; i < nviews; ++i) {
+            float acc = 0.0f;
+            add_view(i, acc);
+            tot += acc;
+        }
+        return tot;
+    }
+    for (int p = 0; p < BP2D_PARTS; ++p) {
+        const int end = part_begin(p + 1, nviews, BP2D_PARTS);
+        float acc = 0.0f;
+        for (int i = part_begin(p, nviews, BP2D_PARTS); i < end; ++i) add_view(i, acc);
+        tot += acc;
+    }
+    return tot;
+}
+
 __device__ __forceinline__ float bp2d_pixel(const float *sino, long long sino_pitch, int row0, int nviews,
                                             const BPView2D *views, int W, int H, int ndet, int R, int kind, int fbp,
                                             int X, int Y)
 {
-    const float sub = 1.0f / (float)R;
-    float tot = 0.0f;
-    for (int p = 0; p < BP2D_PARTS; ++p) {
-        const int end = part_begin(p + 1, nviews, BP2D_PARTS);
-        float acc = 0.0f;
-        for (int i = part_begin(p, nviews, BP2D_PARTS); i < end; ++i) {
-            const BPView2D &C = views[i];
-            const float *row = sino + (long long)(row0 + i) * sino_pitch;
-            for (int ix = 0; ix < R; ++ix) {
-                for (int iy = 0; iy < R; ++iy) {
-                    float x = (float)X - 0.5f * (float)W + 0.5f;
-                    float y = (float)Y - 0.5f * (float)H + 0.5f;
-                    if (R > 1) {
-                        x += -0.5f + 0.5f * sub + (float)ix * sub;
-                        y += -0.5f + 0.5f * sub + (float)iy * sub;
-                    }
-                    if (kind == B2T_GEOM_PAR2D) {
-                        // T - 1/2, T = x c - y s + offset (par_bp.cu:78-81)
-                        const float q = fmaf(x, C.c[0], fmaf(-y, C.c[1], C.c[2] - 0.5f));
-                        acc = fmaf(lerp_line(row, 1, ndet, q), C.c[3], acc);
-                    } else {
-                        // world y is flipped (fan_bp.cu:73)
-                        const float yw = -y;
-                        const float num = fmaf(x, C.c[1], fmaf(yw, C.c[2], C.c[0]));
-                        const float den = fmaf(x, C.c[4], fmaf(yw, C.c[5], C.c[3]));
-                        const float fr = rcp_newton(den);
-                        const float w = fbp ? fr * fr : fr;
-                        acc = fmaf(lerp_line(row, 1, ndet, fmaf(num, fr, -0.5f)), w, acc);
-                    }
-                }
-            }
-        }
-        tot += acc;
-    }
-    return tot;
+    return R == 1 ? bp2d_pixel_sum<true>(sino, sino_pitch, row0, nviews, views, W, H, ndet, 1, kind, fbp, X, Y)
+                  : bp2d_pixel_sum<false>(sino, sino_pitch, row0, nviews, views, W, H, ndet, R, kind, fbp, X, Y);
 }
 
 }  // namespace b2t
