@@ -270,7 +270,7 @@ struct Op2D : Operator {
     }
     b2t_status bp_update(const float *proj, const SirtUpdate2D &u, cudaStream_t s) override
     {
-        if (pix_ss != 1 || g.dims.angles > (uint32_t)BP2D_MAX_VIEWS) return B2T_ERR_UNSUPPORTED;
+        if (pix_ss != 1 || g.dims.angles > (uint32_t)BP2D_MAX_VIEWS || bp2d_few_views(g.dims)) return B2T_ERR_UNSUPPORTED;
         return bp2d_lines(&g, 0, proj, g.dims.dets, nullptr, g.dims.vol_width, B2T_MODE_SET, &u, s);
     }
 };

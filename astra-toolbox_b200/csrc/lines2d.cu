@@ -793,6 +793,22 @@ b2t_status fp2d_lines(const b2t_geom2d *g, uint32_t det_supersample, const float
     return run(g, det_supersample, vol, vol_pitch, sino, sino_pitch, mode, res_b, res_w, s);
 }
 
+// A warp that runs all BP2D_PARTS ranges itself goes through the staging of
+// each of them, and with a view or less a range that is all it does.  Lines and
+// direct kernel (parallel) at 1024^2: 1 view 25.3 and 14.2 us, 8 views 29.4 and 19.5
+// us, 10 views (which the direct kernel sums in parts as well) 31.4 and 31.5 us; at
+// 4096^2 333 and 54, 393 and 240, 403 and 419 us; fan 435 and 262 us (8 views), 450 and
+// 478 us (10).  Images of less than LINES_BP_WARPS tiles leave room on the GPU and
+// wait for the staging longer: 512^2 fan, 10 views 15.1 and 12.8 us, 12 15.5 and 14.7
+// us, 16 17.0 and 19.0 us.  With the ranges split over warps the calls take the
+// same time.
+bool bp2d_few_views(const b2t_dims2d &d)
+{
+    const long long tiles = (long long)((d.vol_width + 31) / 32) * ((d.vol_height + 3) / 4);
+    if (2 * tiles <= LINES_BP_WARPS) return false;
+    return d.angles <= (uint32_t)(tiles <= LINES_BP_WARPS ? 12 : BP2D_PARTS);
+}
+
 b2t_status bp2d_lines(const b2t_geom2d *g, int32_t fbp_weight, const float *sino, size_t sino_pitch, float *vol,
                       size_t vol_pitch, int32_t mode, const SirtUpdate2D *update, cudaStream_t s)
 {

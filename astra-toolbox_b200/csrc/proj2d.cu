@@ -210,7 +210,8 @@ b2t_status bp2d_impl(const b2t_geom2d *g, uint32_t pixel_supersample, int32_t fb
     if (vol_pitch == 0) vol_pitch = d.vol_width;
     if (sino_pitch == 0) sino_pitch = d.dets;
     if (vol_pitch < d.vol_width || sino_pitch < d.dets) return fail(B2T_ERR_INVALID_ARG, "b2t_bp2d: pitch below row length");
-    if (pixel_supersample == 1) return bp2d_lines(g, fbp_weight, sino, sino_pitch, vol, vol_pitch, mode, nullptr, s);
+    if (pixel_supersample == 1 && !bp2d_few_views(d))
+        return bp2d_lines(g, fbp_weight, sino, sino_pitch, vol, vol_pitch, mode, nullptr, s);
     BP2DLaunch *L = new BP2DLaunch;
     L->sino = sino; L->sino_pitch = (long long)sino_pitch; L->vol = vol; L->vol_pitch = (long long)vol_pitch;
     L->W = d.vol_width; L->H = d.vol_height; L->ndet = d.dets; L->rays = pixel_supersample;
