@@ -696,19 +696,47 @@ cudaError_t launch_bp(BP2DLinesLaunch<CAP> &L, float step, cudaStream_t s)
 // the driver copies at every launch).
 constexpr int LINES_SMALL_VIEWS = 256;
 
+// Which lines the rays of the scan march over: of the image's rows, of its
+// columns.  A parallel view's rays share the choice; a fan view's rays make it
+// one by one (fan_ray2d), from |x| and |y| of source to detector, in 32 bits:
+// all alike when both ends of the detector choose so, on the same side and by
+// more than rounding could change.
+struct LineNeed {
+    bool rows = false, cols = false;
+};
+LineNeed lines_needed(const b2t_geom2d *g)
+{
+    LineNeed need;
+    for (uint32_t i = 0; i < g->dims.angles && !(need.rows && need.cols); ++i) {
+        const b2t_view2d &V = g->views[i];
+        if (g->kind == B2T_GEOM_PAR2D) {
+            (std::fabs(V.src[0]) <= std::fabs(V.src[1]) ? need.rows : need.cols) = true;
+            continue;
+        }
+        const double n = (double)g->dims.dets - 1.0;
+        double d[2][2], margin = 1.0;  // [end][axis]
+        for (int k = 0; k < 2; ++k) {
+            for (int e = 0; e < 2; ++e) d[e][k] = e * n * V.det_u[k] + V.det_s[k] + 0.5 - V.src[k];
+            margin += std::fabs((double)V.src[k]) + std::fabs((double)V.det_s[k]) + n * std::fabs((double)V.det_u[k]);
+        }
+        margin *= 1e-5;
+        auto all = [&](int k) {  // every ray is longer along axis k
+            return d[0][k] * d[1][k] > 0.0 && std::fabs(d[0][k]) - std::fabs(d[0][1 - k]) > margin &&
+                   std::fabs(d[1][k]) - std::fabs(d[1][1 - k]) > margin;
+        };
+        if (!all(0)) need.rows = true;
+        if (!all(1)) need.cols = true;
+    }
+    return need;
+}
+
 template <int CAP>
 b2t_status fp_run(const b2t_geom2d *g, uint32_t det_supersample, const float *vol, size_t vol_pitch, float *sino,
                   size_t sino_pitch, int32_t mode, const float *res_b, const float *res_w, cudaStream_t s)
 {
     const b2t_dims2d &d = g->dims;
-    // which lines the rays march over: a parallel view's rays share the
-    // choice, a fan view's rays make it one by one
-    bool rows = false, cols = false;
-    if (g->kind == B2T_GEOM_FAN2D) rows = cols = true;
-    for (uint32_t i = 0; i < d.angles && !(rows && cols); ++i) {
-        if (std::fabs(g->views[i].src[0]) <= std::fabs(g->views[i].src[1])) rows = true;
-        else cols = true;
-    }
+    const LineNeed need = lines_needed(g);
+    const bool rows = need.rows, cols = need.cols;
     size_t total = 0;
     const size_t row_bytes = rows ? lines_bytes(d.vol_height, d.vol_width, total) : 0;
     if (cols) lines_bytes(d.vol_width, d.vol_height, total);
@@ -791,6 +819,23 @@ b2t_status fp2d_lines(const b2t_geom2d *g, uint32_t det_supersample, const float
 {
     auto run = g->dims.angles <= LINES_SMALL_VIEWS ? fp_run<LINES_SMALL_VIEWS> : fp_run<FP2D_MAX_VIEWS>;
     return run(g, det_supersample, vol, vol_pitch, sino, sino_pitch, mode, res_b, res_w, s);
+}
+
+// Calls that the copy into lines, a launch and an allocation, costs more than it
+// gives.  Lines and direct kernel, whole calls: 64^2 and up to 64 views 14.3 to 15.7
+// and 12.3 to 14.6 us; 96^2 parallel, up to 16 views, 15.4 to 16.9 and 14.2 to 15.6 us.
+// One or two fan views whose rays march over rows, where the direct kernel's
+// loads are coalesced: 96^2 and 128^2 14.7 to 15.2 and 12.1 to 13.4 us, 4096^2
+// (the copy is 200 MB) 391 to 395 and 283 to 300 us; between them the lines win (256^2
+// 21 and 23 us, 1024^2 51 and 78 us), as they do where rays march over columns (4096^2
+// 398 and 1055 us).
+bool fp2d_few_rays(const b2t_geom2d *g)
+{
+    const b2t_dims2d &d = g->dims;
+    const uint32_t n = std::max(d.vol_width, d.vol_height);
+    if (n <= 64 && d.angles <= 64) return true;
+    if (g->kind == B2T_GEOM_PAR2D) return n <= 96 && d.angles <= 16;
+    return d.angles <= 2 && (n <= 128 || n >= 4096) && !lines_needed(g).cols;
 }
 
 // A warp that runs all BP2D_PARTS ranges itself goes through the staging of

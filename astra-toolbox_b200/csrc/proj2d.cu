@@ -149,9 +149,11 @@ b2t_status fp2d_impl(const b2t_geom2d *g, uint32_t det_supersample, const float 
     if (vol_pitch == 0) vol_pitch = d.vol_width;
     if (sino_pitch == 0) sino_pitch = d.dets;
     if (vol_pitch < d.vol_width || sino_pitch < d.dets) return fail(B2T_ERR_INVALID_ARG, "b2t_fp2d: pitch below row length");
-    const b2t_status st = fp2d_lines(g, det_supersample, vol, vol_pitch, sino, sino_pitch, mode, nullptr, nullptr, s);
-    if (st != B2T_ERR_NO_MEMORY) return st;
-    clear_error();
+    if (!fp2d_few_rays(g)) {
+        const b2t_status st = fp2d_lines(g, det_supersample, vol, vol_pitch, sino, sino_pitch, mode, nullptr, nullptr, s);
+        if (st != B2T_ERR_NO_MEMORY) return st;
+        clear_error();
+    }
     const int acc = (mode == B2T_MODE_ADD) ? 1 : 0;
     if (g->kind == B2T_GEOM_PAR2D) {
         FP2DParLaunch *L = new FP2DParLaunch;

@@ -86,7 +86,9 @@ b2t_status fp2d_lines(const b2t_geom2d *g, uint32_t det_supersample, const float
 b2t_status bp2d_lines(const b2t_geom2d *g, int32_t fbp_weight, const float *sino, size_t sino_pitch, float *vol,
                       size_t vol_pitch, int32_t mode, const SirtUpdate2D *update, cudaStream_t s);
 
-// Whether a backprojection has so few views that the direct kernel is faster.
+// Whether a projection has so few rays that the direct kernel is faster, and a
+// backprojection so few views.
+bool fp2d_few_rays(const b2t_geom2d *g);
 bool bp2d_few_views(const b2t_dims2d &d);
 
 b2t_status validate2d(const b2t_geom2d *g, const char *who);

@@ -1,5 +1,9 @@
-"""2D backprojections of few views, which run the direct kernel, at the edges
-of the rule: the values of the oracle and of a longer scan's first views."""
+"""2D calls with few views or few rays, which run the direct kernels, at the
+edges of both rules: the values of the line kernels (whose bits they share), of
+the oracle, and of a longer scan's first views; fan scans whose rays march over
+rows, over columns, over both."""
+import importlib
+
 import numpy as np
 import pytest
 
@@ -16,6 +20,10 @@ def _geom(astra, kind, rows, cols, views, start=0.1, total=None):
     if kind == 'parallel':
         return astra.create_proj_geom('parallel', 1.0, int(1.4 * n), ang), vg
     return astra.create_proj_geom('fanflat', 1.5, int(1.4 * n), ang, 2.0 * n, 1.0 * n), vg
+
+
+def _launches():
+    return importlib.import_module("astra-toolbox_b200._lib").load().b2t_kernel_launches()
 
 
 # backprojection: images of one warp a tile (more than 1800 tiles of 32 x 4), of
@@ -44,6 +52,40 @@ def test_bp_equals_the_views_of_a_longer_scan(astra, orc, kind, n):
             # positions of up to 350 texels, rounded twice, move by up to 2^-16 texels
             # each, and a sample of this noise by as much as its own size per texel
             assert rel_l2(a.cpu().numpy(), ref) < 2 * 2 ** -16
+
+
+@pytest.mark.parametrize("kind", ["parallel", "fanflat"])
+@pytest.mark.parametrize("rows,cols", [(64, 64), (64, 65), (65, 30), (96, 80), (97, 97), (128, 100), (129, 128)])
+def test_fp_against_the_oracle(astra, orc, kind, rows, cols):
+    """Launches tell the direct kernel (one) from the lines (two)."""
+    for views in (1, 2, 3, 16, 17, 64, 65):
+        for start in (0.1, 0.78, 1.6):
+            pg, vg = _geom(astra, kind, rows, cols, views, start, total=max(views, 50))
+            pr = astra.Projector2D(pg, vg)
+            vol = torch.rand(pr.vol_shape, device='cuda')
+            n = _launches()
+            fp = pr.fp(vol, torch.zeros(pr.proj_shape, device='cuda'))
+            n = _launches() - n
+            big = max(rows, cols)
+            few = views <= 16 and big <= 96 if kind == 'parallel' else views <= 2 and big <= 128 and start == 0.1
+            direct = big <= 64 and views <= 64 or few
+            assert n == (1 if direct else 2), (views, start, n)
+            ref = (orc.fan_fp if kind == 'fanflat' else orc.par_fp)(pr.geom.views_array(), vol.cpu().numpy(),
+                                                                    pr.proj_shape[1], pr.geom.output_scale, rays=1)
+            assert rel_l2(fp.cpu().numpy(), ref) < 1e-5
+
+
+@pytest.mark.parametrize("start", np.linspace(0.0, 1.6, 17))
+def test_fan_scans_with_one_set_of_lines(astra, orc, start):
+    """Three neighbouring views, whose rays march over rows, over columns or over both,
+    with and without supersampling."""
+    pg, vg = _geom(astra, 'fanflat', 150, 131, 3, start, total=360)
+    for rays in (1, 3):
+        pr = astra.Projector2D(pg, vg, {'DetectorSuperSampling': rays})
+        vol = torch.rand(pr.vol_shape, device='cuda')
+        fp = pr.fp(vol, torch.zeros(pr.proj_shape, device='cuda'))
+        ref = orc.fan_fp(pr.geom.views_array(), vol.cpu().numpy(), pr.proj_shape[1], pr.geom.output_scale, rays=rays)
+        assert rel_l2(fp.cpu().numpy(), ref) < 1e-5
 
 
 def test_sirt_of_few_views(astra, orc):
