@@ -727,7 +727,8 @@ b2t_status fp3d_cells_build(const b2t_geom3d *g, const b2t_params3d *p, const vo
     std::vector<int> dirs(g->dims.angles);
     for (uint32_t a = 0; a < g->dims.angles; ++a) dirs[a] = dominant_axis(g->kind, g->views[a], g->dims);
     bool slab[3] = {false, false, false};
-    for (int dir = 0; dir < 2; ++dir) slab[dir] = need[dir] && fp_slab_eligible(g, p, dir, dirs);
+    for (int dir = 0; dir < 2; ++dir)
+        slab[dir] = need[dir] && (dtype == B2T_F32 || fp_slab_pays(g, dir, dirs)) && fp_slab_eligible(g, p, dir, dirs);
     if (dtype == B2T_F32) return build_cells_t<float>(g, vol, vol_pitch, need, slab, s, c);
     if (dtype == B2T_F16) return build_cells_t<__half>(g, vol, vol_pitch, need, slab, s, c);
     return build_cells_t<__nv_bfloat16>(g, vol, vol_pitch, need, slab, s, c);

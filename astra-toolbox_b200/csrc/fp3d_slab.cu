@@ -104,6 +104,20 @@ static_assert((SLAB_SLOT * 8) % 128 == 0 && (SLAB_BOX_Y * SLAB_WA * 8) % 128 == 
 static_assert(32 % SLAB_PER == 0, "a producer batch is made of whole stages");
 static_assert(4 * SLAB_W <= 32, "the producer projects the corner rays one per lane");
 
+// Whether a box of ny x nz texels fits a slice buffer.
+__host__ __device__ constexpr bool slab_fits(int ny, int nz)
+{
+    return nz <= SLAB_WB &&
+           ((ny + SLAB_BOX_Y - 1) / SLAB_BOX_Y) * SLAB_BOX_Y * (nz <= SLAB_WA ? SLAB_WA : SLAB_WB) <= SLAB_SLOT;
+}
+
+// Detector rows of a CTA: the fewest row blocks, of equal height.
+int slab_rows(const b2t_dims3d &d)
+{
+    const int blocks = (int)((d.det_v + SLAB_ROWS - 1) / SLAB_ROWS);
+    return 32 * (((int)d.det_v + 32 * blocks - 1) / (32 * blocks));
+}
+
 // The launch record of the FP and of its transpose (bp3d_slab_matched_kernel,
 // which reads the projections and writes the accumulator through tmap / acc).
 struct alignas(64) SlabLaunch {
@@ -293,8 +307,7 @@ __device__ __noinline__ void slab_produce(const SlabLaunch &L, float2 *buf, uint
             z0 = ((zlo + 2) & ~1) - 2;  // TMA: (z0 + 2) * 8 bytes on a 16-byte boundary
             ny = y1 - y0 + 1;
             nz = z1 - z0 + 1;
-            fit = C.hull && sane && nz <= SLAB_WB &&
-                  ((ny + SLAB_BOX_Y - 1) / SLAB_BOX_Y) * SLAB_BOX_Y * (nz <= SLAB_WA ? SLAB_WA : SLAB_WB) <= SLAB_SLOT;
+            fit = C.hull && sane && slab_fits(ny, nz);
         };
         measure(slab_box<false>(L, C, (float)(s_lo + b0 + lane), y0, y1, zlo, z1));
         const bool whole = fit;
@@ -1091,10 +1104,12 @@ __global__ void __launch_bounds__(256) build_slab_copy(const T *__restrict__ vol
     }
 }
 
-bool slab_enabled()
+// B2T_FP_PATH=cells keeps the cell kernels for every view, =slab takes the slab
+// kernel for every view that it can (16-bit data whether it pays or not).
+bool slab_path(char c)
 {
     const char *e = std::getenv("B2T_FP_PATH");
-    return !(e && e[0] == 'c');  // B2T_FP_PATH=cells keeps the cell kernels for every view
+    return e && e[0] == c;
 }
 
 long long slab_pz(const b2t_dims3d &d) { return ((long long)d.vol_z + 4 + 1) & ~1ll; }
@@ -1128,7 +1143,7 @@ b2t_status fp_slab_errors(uint32_t *flags)
 
 bool fp_slab_eligible(const b2t_geom3d *g, const b2t_params3d *p, int dir, const std::vector<int> &dirs)
 {
-    if (!slab_enabled() || dir > 1 || p->det_supersample != 1) return false;
+    if (slab_path('c') || dir > 1 || p->det_supersample != 1) return false;
     const b2t_dims3d &d = g->dims;
     if (d.vol_y + 4 > 65535) return false;  // (the copy's grid)
     for (uint32_t a = 0; a < d.angles; ++a) {
@@ -1138,6 +1153,107 @@ bool fp_slab_eligible(const b2t_geom3d *g, const b2t_params3d *p, int dir, const
         if (w.e[2] != 0.0f || w.m1[2] != 0.0f || w.n1[2] != 0.0f) return false;
     }
     return true;
+}
+
+// 16-bit data: the cell kernels read two bytes a texel where the slab reads FP32
+// pairs, and beat it where its CTAs are few, hold few rows, read global memory
+// or follow rays that have left the volume.  Slab over cells, FP16:
+//  - waves of CTAs in the launch (two an SM), PAY_WAVES or, of CTAs of PAY_TALL rows
+//    whose boxes nearly all fit, PAY_TALL_WAVES: 256^3 x 24 views 2.1 waves 1.28, 128^3
+//    x 90 (96 rows) 2.8 1.12, 200^3 x 45 2.3 1.02, 96^3 x 180 (160 rows) 2.1 1.04, 128^3 x
+//    180 (parallel, 160 rows) 2.3 0.93, 198^2 x 104 x 138 (128 rows) 2.7 0.78, 160^3 x 90
+//    3.4 0.95, 200^3 x 90 4.4 0.85, 256^3 x 180 16 0.80;
+//  - PAY_ROWS a CTA: a 256^3 volume x 360 views on 32 detector rows (11 waves) 1.78, 64
+//    rows 1.10, 96 (two blocks of them) 0.86 to 0.95, 128 to 160 0.69 to 0.87;
+//  - PAY_FIT, the share of slice boxes that fit a buffer (neighbouring views far
+//    apart, magnified or coarse detectors): 0.65 (spacing 1.6 texels) 1.38, 0.83 (320^3 x
+//    90) 0.89, 0.87 (256^3, magnified five times) 0.96, 320^3 x 45 1.11, above that as
+//    the rows say;
+//  - PAY_USE, the share of a box inside the volume: a source three quarters of a
+//    128^3 volume's width away 0.74 1.08, 256^3 and 0.6 pixels 0.8 0.73.
+// The shares are those of a sample: up to six pairs of neighbouring views (less
+// the worst, a pair on either side of the other direction's views), three
+// columns of tiles, the first and the middle row of them, five slices.  About 7 us
+// of host time, asked only of launches of PAY_TALL_WAVES, several hundred us.
+constexpr double PAY_WAVES = 3.5, PAY_FIT = 0.9, PAY_USE = 0.75, PAY_TALL_WAVES = 2.2, PAY_TALL_FIT = 0.99;
+constexpr int PAY_ROWS = 96, PAY_TALL = 128;
+
+bool fp_slab_pays(const b2t_geom3d *g, int dir, const std::vector<int> &dirs)
+{
+    if (slab_path('s')) return true;
+    const b2t_dims3d &d = g->dims;
+    const int rows = slab_rows(d);
+    if (rows < PAY_ROWS) return false;
+    std::vector<uint32_t> views;
+    for (uint32_t a = 0; a < d.angles; ++a)
+        if (dirs[a] == dir) views.push_back(a);
+    const int pairs = (int)(views.size() + SLAB_W - 1) / SLAB_W;
+    const int nub = ((int)d.det_u + SLAB_U - 1) / SLAB_U, nvb = ((int)d.det_v + rows - 1) / rows;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    const double waves = (double)pairs * nub * nvb / (2 * sms);
+    if (waves < (rows >= PAY_TALL ? PAY_TALL_WAVES : PAY_WAVES)) return false;
+    const int n0 = (int)(dir == 0 ? d.vol_x : d.vol_y), n1 = (int)(dir == 0 ? d.vol_y : d.vol_x), n2 = (int)d.vol_z;
+    const int samples = std::min(pairs, 6);
+    double worst = 1.0, fit = 0.0, use = 0.0;
+    for (int k = 0; k < samples; ++k) {
+        const int first = SLAB_W * (int)((2LL * k + 1) * pairs / (2 * samples));
+        FPView w[SLAB_W];
+        for (int i = 0; i < SLAB_W; ++i)
+            fp_view_coeffs(g->kind, g->views[views[std::min(first + i, (int)views.size() - 1)]], d, dir, w[i]);
+        int met = 0, fits = 0;
+        double inside = 0.0;
+        for (int t = 0; t < 6; ++t) {
+            const int u0 = SLAB_U * (nub * (t / 2 + 1) / 4), v0 = rows * (t % 2 ? nvb / 2 : 0);
+            double A1[SLAB_NC], B1[SLAB_NC], A2[SLAB_NC], B2[SLAB_NC];
+            for (int c = 0; c < SLAB_NC; ++c) {
+                const FPView &V = w[c >> 2];
+                const double uu = std::min(u0 + (c & 1 ? SLAB_U - 1 : 0), (int)d.det_u - 1) + 0.5 - 0.5 * d.det_u;
+                const double vv = std::min(v0 + (c & 2 ? rows - 1 : 0), (int)d.det_v - 1) + 0.5 - 0.5 * d.det_v;
+                const double inv = 1.0 / (V.e[0] + uu * V.e[1]);
+                A1[c] = (V.m1[0] + uu * V.m1[1]) * inv;
+                B1[c] = (V.n1[0] + uu * V.n1[1]) * inv + 0.5;
+                A2[c] = (V.m2[0] + uu * V.m2[1] + vv * V.m2[2]) * inv;
+                B2[c] = (V.n2[0] + uu * V.n2[1] + vv * V.n2[2]) * inv + 0.5;
+            }
+            for (int j = 0; j <= 4; ++j) {
+                const double s = (double)((n0 - 1) * j / 4);
+                double q[4] = {1e9, -1e9, 1e9, -1e9};  // smallest and largest positions
+                for (int c = 0; c < SLAB_NC; ++c) {
+                    const double q1 = A1[c] * s + B1[c], q2 = A2[c] * s + B2[c];
+                    q[0] = std::min(q[0], q1);
+                    q[1] = std::max(q[1], q1);
+                    q[2] = std::min(q[2], q2);
+                    q[3] = std::max(q[3], q2);
+                }
+                if (!(q[1] >= -2.0 && q[0] <= n1 + 1.0 && q[3] >= -2.0 && q[2] <= n2 + 1.0)) continue;
+                ++met;
+                auto texels = [&](bool clamp) {
+                    int e[4];
+                    for (int i = 0; i < 4; ++i) {
+                        const int n = i < 2 ? n1 : n2;
+                        double k1 = std::floor(std::min(std::max(q[i], -1e6), 1e6)) + (i & 1 ? 2.0 : -1.0);
+                        if (clamp) k1 = std::min(std::max(k1, -2.0), n + 1.0);
+                        e[i] = (int)k1;
+                    }
+                    return slab_fits(e[1] - e[0] + 1, e[3] - (((e[2] + 2) & ~1) - 2) + 1);
+                };
+                fits += texels(false) || texels(true);
+                inside += std::max(0.0, std::min(q[3], n2 + 1.0) - std::max(q[2], -1.0)) / std::max(q[3] - q[2], 1e-9);
+            }
+        }
+        if (met == 0) met = fits = 1;
+        const double f = (double)fits / met;
+        worst = std::min(worst, f);
+        fit += f;
+        use += inside / met;
+    }
+    if (samples > 1) fit = (fit - worst) / (samples - 1);
+    return fit >= (waves < PAY_WAVES ? PAY_TALL_FIT : PAY_FIT) && use / samples >= PAY_USE;
 }
 
 size_t fp_slab_copy_bytes(const b2t_dims3d &d, int dir)
@@ -1204,9 +1320,7 @@ b2t_status fp_slab_project(const b2t_geom3d *g, const b2t_params3d *p, const voi
     L.nv = d.det_v;
     L.na = d.angles;
     L.accumulate = (mode == B2T_MODE_ADD) ? 1 : 0;
-    // the fewest row blocks, of equal height
-    const int blocks = (int)((d.det_v + SLAB_ROWS - 1) / SLAB_ROWS);
-    L.rows = 32 * (((int)d.det_v + 32 * blocks - 1) / (32 * blocks));
+    L.rows = slab_rows(d);
     fp_scale(g->kind, dir, g->vol_scale, false, p->output_scale, L.f1, L.f2, L.mul);
     std::vector<int> views;
     for (uint32_t a = 0; a < d.angles; ++a)

@@ -154,6 +154,8 @@ b2t_status fp3d_cells_build(const b2t_geom3d *g, const b2t_params3d *p, const vo
 // whose rays share the in-plane position along a detector column, any storage
 // type, no detector supersampling.
 bool fp_slab_eligible(const b2t_geom3d *g, const b2t_params3d *p, int dir, const std::vector<int> &dirs);
+// Whether it is faster than the cell kernels for 16-bit data (for FP32 it always is).
+bool fp_slab_pays(const b2t_geom3d *g, int dir, const std::vector<int> &dirs);
 size_t fp_slab_copy_bytes(const b2t_dims3d &d, int dir);
 b2t_status fp_slab_build(const b2t_dims3d &d, const void *vol, size_t vol_pitch, int32_t dtype, int dir, void *copy,
                          cudaStream_t s);

@@ -52,7 +52,8 @@ def test_row_blocks_and_stages(astra, rows, vol, kind, monkeypatch):
 
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
 @pytest.mark.parametrize("kind", ["cone", "parallel3d"])
-def test_16_bit_storage_rounds_the_fp32_projection(astra, dtype, kind):
+def test_16_bit_storage_rounds_the_fp32_projection(astra, dtype, kind, monkeypatch):
+    monkeypatch.setenv("B2T_FP_PATH", "slab")  # (so few views are faster from cells)
     L = importlib.import_module("astra-toolbox_b200._lib")
     t = getattr(torch, dtype)
     ang = np.linspace(0, 2 * np.pi, 25, endpoint=False).astype(np.float32)
@@ -75,3 +76,49 @@ def test_16_bit_storage_rounds_the_fp32_projection(astra, dtype, kind):
     add = base.clone()
     pr.fp(tv, add, mode=0)
     assert torch.equal(add, (full + base.float()).to(t))
+
+
+# (views, detector columns, rows, volume, slab): enough CTAs of enough rows; too
+# few CTAs, too few rows in each, neighbouring views too far apart for a slice
+# buffer, a source so close that the rays of a CTA leave the volume one by one
+CHOICES = {
+    "many": (430, 110, 90, (64, 64, 70), 1.2, 2.0, True),
+    "tall": (220, 130, 125, (90, 90, 100), 1.2, 2.0, True),
+    "few_views": (120, 110, 90, (64, 64, 70), 1.2, 2.0, False),
+    "few_rows": (430, 110, 60, (64, 64, 40), 1.2, 2.0, False),
+    "far_views": (44, 900, 150, (300, 300, 100), 0.6, 2.0, False),
+    "near_source": (430, 110, 130, (64, 64, 64), 5.0, 0.75, False),
+}
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("case", list(CHOICES))
+def test_16_bit_choice_of_kernel(astra, case, dtype, monkeypatch):
+    """Which 16-bit scans take the slab, with the other choice's values; FP32
+    ones all do."""
+    L = importlib.import_module("astra-toolbox_b200._lib")
+    views, nu, nv, (ny, nx, nz), px, so, slab = CHOICES[case]
+    ang = np.linspace(0, 2 * np.pi, views, endpoint=False).astype(np.float32)
+    od = 3.0 if so < 1 else 1.0
+    pg = astra.create_proj_geom('cone', px, px, nv, nu, ang, so * nx, od * nx)
+    pr = astra.Projector3D(pg, astra.create_vol_geom(ny, nx, nz))
+    t = getattr(torch, dtype)
+    vol = torch.rand(pr.vol_shape, device='cuda', generator=torch.Generator('cuda').manual_seed(1)).to(t)
+    out = {}
+    for path in (None, "cells", "slab"):
+        if path:
+            monkeypatch.setenv("B2T_FP_PATH", path)
+        _stats(L)
+        out[path] = torch.zeros(pr.proj_shape, device='cuda', dtype=t)
+        pr.fp(vol, out[path])
+        s = _stats(L)
+        assert (s[2] > 0, s[3] > 0) == ((False, True) if path == "cells" or not (path or slab) else (True, False))
+    monkeypatch.delenv("B2T_FP_PATH")
+    assert torch.equal(out[None], out["slab" if slab else "cells"])
+    # one rounding of the output; the cells hold 16-bit differences as well
+    tol = {"float16": 1e-3, "bfloat16": 8e-3}[dtype]
+    assert rel_l2(out["cells"].float().cpu().numpy(), out["slab"].float().cpu().numpy()) < tol
+    full = torch.zeros(pr.proj_shape, device='cuda')
+    _stats(L)
+    pr.fp(vol.float(), full)
+    assert _stats(L)[3] == 0
