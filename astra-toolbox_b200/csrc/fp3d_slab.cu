@@ -694,8 +694,8 @@ __global__ void __launch_bounds__(SLAB_THREADS, 2) fp3d_slab_kernel(const __grid
 // issues 4 reductions), while the same kernel with 32-bit integer reductions
 // at the same addresses takes 29.9 ms and with plain stores 16.8 ms, which
 // bounds any shared-memory accumulation of this tiling at 0.72x of the
-// scatter.  So the scatter kernels stay the default and this kernel runs
-// only when B2T_MATCHED_PATH=slab selects it.
+// scatter.  So the scatter and the gather (matched_gather.cu) are what calls
+// use and this kernel runs only when B2T_MATCHED_PATH=slab selects it.
 //
 // A tap lands inside its box for the reason an FP sample reads inside it:
 // at a slice, the rays of a detector rectangle whose denominators share a
@@ -1354,7 +1354,8 @@ static std::atomic<unsigned long long> g_mt_launches{0};
 bool matched_slab_eligible(const b2t_geom3d *g, const b2t_params3d *p, int dir, const std::vector<int> &dirs)
 {
     // opt-in (B2T_MATCHED_PATH=slab): the per-sample global reductions of
-    // matched.cu are faster on this hardware, see the kernel's comment
+    // matched.cu and the gather are faster on this hardware, see the kernel's
+    // comment
     const char *e = std::getenv("B2T_MATCHED_PATH");
     if (!(e && std::string(e) == "slab") || dir > 1 || p->det_supersample != 1) return false;
     const b2t_dims3d &d = g->dims;
@@ -1460,7 +1461,9 @@ b2t_status matched_path_stats_impl(uint64_t *stats)
     stats[0] = v[0];
     stats[1] = v[1];
     stats[2] = g_mt_launches.exchange(0);
-    stats[3] = matched_scatter_launches_take();
+    unsigned long long scatters = 0;
+    B2T_TRY(matched_scatter_launches_take(&scatters));
+    stats[3] = scatters;
     return B2T_OK;
 }
 

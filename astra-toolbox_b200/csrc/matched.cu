@@ -164,6 +164,7 @@ __device__ __forceinline__ void red_add_v4(float4 *p, float a, float b, float c,
 template <typename T, bool AGG>
 __global__ void __launch_bounds__(256) fp3d_transpose_cols_kernel(const __grid_constant__ FPLaunch L)
 {
+    if (L.gathered && *L.gathered) return;
     const FPView &V = L.views[blockIdx.x];
     const int v = blockIdx.z * 32 + threadIdx.x;
     const int u = blockIdx.y * 8 + threadIdx.y;
@@ -288,27 +289,29 @@ template <typename T>
 __global__ void fold_cells(const float4 *__restrict__ c0, const float4 *__restrict__ c1,
                            const float *__restrict__ accA, const float *__restrict__ m0,
                            const float *__restrict__ m1, long long ay0, long long ay1, long long az, int nx, int ny,
-                           int nz, T *__restrict__ out, size_t pitch, int accumulate)
+                           int nz, T *__restrict__ out, size_t pitch, int accumulate, const int *__restrict__ gathered)
 {
+    if (gathered && *gathered) return;
     const int z = blockIdx.x * blockDim.x + threadIdx.x;
-    const int x = blockIdx.y;
     const int y = blockIdx.z;
     if (z >= nz) return;
     const long long m2 = nz + 4;
-    float r = 0.0f;
-    auto taps = [&](const float4 *c, long long j1, long long n0, long long sl) {
-        const float4 *p = c + (j1 * n0 + sl) * m2 + (z + 2);  // cell (k1, s, k2 = z)
-        const float4 *q = p - n0 * m2;                        // k1 - 1
-        r += p->x + q->y + (p - 1)->z + (q - 1)->w;
-    };
-    if (c0) taps(c0, y + 2, nx, x);
-    if (c1) taps(c1, x + 2, ny, y);
-    if (accA) r += accA[((size_t)(z + 2) * (ny + 4) + (y + 2)) * (nx + 4) + (x + 2)];
-    if (m0) r += m0[((long long)x * ay0 + y + 2) * az + z + 2];
-    if (m1) r += m1[((long long)y * ay1 + x + 2) * az + z + 2];
-    T *o = out + ((size_t)z * ny + y) * pitch + x;
-    if (accumulate) r += ldm_plain(o);
-    *o = tom<T>(r);
+    for (int x = blockIdx.y; x < nx; x += gridDim.y) {
+        float r = 0.0f;
+        auto taps = [&](const float4 *c, long long j1, long long n0, long long sl) {
+            const float4 *p = c + (j1 * n0 + sl) * m2 + (z + 2);  // cell (k1, s, k2 = z)
+            const float4 *q = p - n0 * m2;                        // k1 - 1
+            r += p->x + q->y + (p - 1)->z + (q - 1)->w;
+        };
+        if (c0) taps(c0, y + 2, nx, x);
+        if (c1) taps(c1, x + 2, ny, y);
+        if (accA) r += accA[((size_t)(z + 2) * (ny + 4) + (y + 2)) * (nx + 4) + (x + 2)];
+        if (m0) r += m0[((long long)x * ay0 + y + 2) * az + z + 2];
+        if (m1) r += m1[((long long)y * ay1 + x + 2) * az + z + 2];
+        T *o = out + ((size_t)z * ny + y) * pitch + x;
+        if (accumulate) r += ldm_plain(o);
+        *o = tom<T>(r);
+    }
 }
 
 // out[z][y][x] (=|+=) accA[z+2][y+2][x+2] + accB[z+2][x+2][y+2]
@@ -329,10 +332,59 @@ __global__ void fold_accumulators(const float *__restrict__ accA, const float *_
     *o = tom<T>(r);
 }
 
+// Gather or scatter, where the geometry suits both (matched_gather.cu): the
+// scatter skips rays without a value, the gather only whole columns without one,
+// and 256^3 x 360 views take 19.0 ms scattered and 16.1 ms gathered on dense
+// projections, but 6.0 and 11.3 ms on those of an ellipsoid that leaves half of
+// the rays empty.  So the gather runs when at least nine rays in ten of a sample
+// hold a value, and the host enqueues both: it would have to wait for the
+// projections to choose.  One block, four samples a thread, spread evenly over
+// rows and columns by a two-dimensional Kronecker sequence (the share is within
+// 1 % of all rays').
+// What does not run costs its empty blocks: of 192^3 x 240 views the scatter 60 us
+// beside a gather of 4.5 ms, the gather 20 us beside a scatter of 0.7 to 5.3 ms.
+constexpr int CHOOSE_THREADS = 1024, CHOOSE_SAMPLES = 4;
+__device__ unsigned long long g_scatters_chosen = 0;
+
+template <typename T>
+__global__ void __launch_bounds__(CHOOSE_THREADS) matched_choose_kernel(const T *__restrict__ proj, long long pitch,
+                                                                        unsigned nu, unsigned long long rows,
+                                                                        int scatters, int *gathered)
+{
+    int held = 0;
+#pragma unroll
+    for (int k = 0; k < CHOOSE_SAMPLES; ++k) {
+        // 2^32 over the plastic number and over its square
+        const uint32_t n = threadIdx.x * CHOOSE_SAMPLES + k, hu = n * 3242174889u, hv = n * 2447445414u;
+        const unsigned long long row = __umul64hi((unsigned long long)hv << 32, rows);
+        held += ldm(proj + (long long)row * pitch + __umulhi(hu, nu)) != 0.0f;
+    }
+    __shared__ int total;
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    held = __reduce_add_sync(0xffffffffu, held);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&total, held);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    const bool g = 10 * total >= 9 * CHOOSE_THREADS * CHOOSE_SAMPLES;
+    *gathered = g;
+    if (!g) atomicAdd(&g_scatters_chosen, (unsigned long long)scatters);
+}
+
+// n float4 zeros unless the gather runs.
+__global__ void clear_cells(float4 *p, size_t n, const int *__restrict__ gathered)
+{
+    if (*gathered) return;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        p[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+}
+
+// Scatter launches enqueued without a choice.
+std::atomic<unsigned long long> g_scatter_launches{0};
+
 // B2T_MATCHED_PLAIN=1 selects the per-lane reductions of
 // fp3d_transpose_cols_kernel (the path of arrays of 2^32 cells or more)
 // instead of the merged ones (same sums, another order; tests compare them).
-std::atomic<unsigned long long> g_scatter_launches{0};
 
 bool matched_force_plain()
 {
@@ -363,7 +415,21 @@ b2t_status launch_fold(const float *a, const float *b, const b2t_dims3d &d, void
 
 }  // namespace
 
-unsigned long long matched_scatter_launches_take() { return g_scatter_launches.exchange(0); }
+b2t_status matched_scatter_launches_take(unsigned long long *n)
+{
+    unsigned long long v = 0;
+    B2T_CUDA_TRY(cudaMemcpyFromSymbol(&v, g_scatters_chosen, sizeof(v)), "read matched BP path statistics");
+    const unsigned long long zero = 0;
+    B2T_CUDA_TRY(cudaMemcpyToSymbol(g_scatters_chosen, &zero, sizeof(zero)), "clear matched BP path statistics");
+    *n = v + g_scatter_launches.exchange(0);
+    return B2T_OK;
+}
+
+std::string matched_path_env()
+{
+    const char *e = std::getenv("B2T_MATCHED_PATH");
+    return e ? e : "";
+}
 
 b2t_status matched_bp3d_impl(const b2t_geom3d *g, const b2t_params3d *p, const void *proj,
                              size_t proj_pitch, void *vol, size_t vol_pitch, int32_t dtype,
@@ -377,21 +443,32 @@ b2t_status matched_bp3d_impl(const b2t_geom3d *g, const b2t_params3d *p, const v
     if (vol_pitch < d.vol_x || proj_pitch < d.det_u)
         return fail(B2T_ERR_INVALID_ARG, "b2t_bp3d(matched): pitch below row length");
     std::vector<int> dirs(d.angles);
+    std::vector<FPView> coeffs(d.angles);
     bool need[3] = {false, false, false};
     for (uint32_t a = 0; a < d.angles; ++a) {
         dirs[a] = dominant_axis(g->kind, g->views[a], d);
         need[dirs[a]] = true;
+        fp_view_coeffs(g->kind, g->views[a], d, dirs[a], coeffs[a]);
+        coeffs[a].a = (int)a;
     }
-    // gathered per voxel where every view allows it (matched_gather.cu), else
-    // scattered; without memory for its weighted rows, scattered as well
-    const bool slab_asked =
-        (need[0] && matched_slab_eligible(g, p, 0, dirs)) || (need[1] && matched_slab_eligible(g, p, 1, dirs));
-    if (!slab_asked && !matched_force_plain() && matched_gather_eligible(g, p, dirs)) {
-        const b2t_status st = matched_gather(g, p, proj, proj_pitch, vol, vol_pitch, dtype,
-                                             (mode == B2T_MODE_ADD) ? 1 : 0, dirs, s);
+    const int accumulate = (mode == B2T_MODE_ADD) ? 1 : 0;
+    // gathered per voxel where every view allows it and it pays
+    // (matched_gather.cu), else scattered; without memory for its weighted
+    // rows, scattered as well
+    const std::string path = matched_path_env();
+    const bool can_gather = (path.empty() || path == "gather") && !matched_force_plain() &&
+                            matched_gather_eligible(g, p, dirs, coeffs, path.empty());
+    auto gather = [&](const int *run) {
+        const b2t_status st = matched_gather(g, p, proj, proj_pitch, vol, vol_pitch, dtype, accumulate, dirs, coeffs, run, s);
+        if (st == B2T_ERR_NO_MEMORY) clear_error();
+        return st;
+    };
+    if (can_gather && path == "gather") {  // (tests)
+        const b2t_status st = gather(nullptr);
         if (st != B2T_ERR_NO_MEMORY) return st;
-        clear_error();
     }
+    Scratch choice;
+    const int *gathered = nullptr;
     const size_t px = d.vol_x + 4, py = d.vol_y + 4, pz = d.vol_z + 4;
     const size_t padded = px * py * pz;
     {
@@ -424,7 +501,39 @@ b2t_status matched_bp3d_impl(const b2t_geom3d *g, const b2t_params3d *p, const v
                 break;
             }
             B2T_TRY(st);
-            B2T_CUDA_TRY(cudaMemsetAsync(cacc[dir].as<void>(), 0, count * sizeof(float4), s), "matched bp memset");
+        }
+        if (ok && can_gather && path.empty()) {
+            b2t_status st = choice.alloc(sizeof(int), s, "matched bp choice");
+            if (st == B2T_OK) {
+                int scatters = 0;
+                for (int dir = 0; dir < 2; ++dir)
+                    scatters += (int)((std::count(dirs.begin(), dirs.end(), dir) + FP_MAX_VIEWS - 1) / FP_MAX_VIEWS);
+                auto choose = [&](auto *y) {
+                    matched_choose_kernel<<<1, CHOOSE_THREADS, 0, s>>>(y, (long long)proj_pitch, d.det_u,
+                                                                       (unsigned long long)d.det_v * d.angles, scatters,
+                                                                       choice.as<int>());
+                };
+                if (dtype == B2T_F32) choose(static_cast<const float *>(proj));
+                else if (dtype == B2T_F16) choose(static_cast<const __half *>(proj));
+                else choose(static_cast<const __nv_bfloat16 *>(proj));
+                count_launches(1);
+                B2T_CUDA_TRY(cudaGetLastError(), "matched bp choice launch");
+                st = gather(choice.as<int>());
+                if (st == B2T_OK) gathered = choice.as<int>();
+            } else if (st == B2T_ERR_NO_MEMORY) {
+                clear_error();
+            }
+            if (st != B2T_ERR_NO_MEMORY) B2T_TRY(st);
+        }
+        for (int dir = 0; dir < 2 && ok; ++dir) {
+            if (!cacc[dir].as<void>()) continue;
+            if (gathered) {
+                clear_cells<<<1184, 256, 0, s>>>(cacc[dir].as<float4>(), cacc[dir].bytes() / sizeof(float4), gathered);
+                count_launches(1);
+                B2T_CUDA_TRY(cudaGetLastError(), "matched bp clear launch");
+            } else {
+                B2T_CUDA_TRY(cudaMemsetAsync(cacc[dir].as<void>(), 0, cacc[dir].bytes(), s), "matched bp memset");
+            }
         }
         if (ok && need[2]) {
             const b2t_status st = sz.alloc(padded * sizeof(float), s, "matched bp accumulator (xyz)");
@@ -454,6 +563,7 @@ b2t_status matched_bp3d_impl(const b2t_geom3d *g, const b2t_params3d *p, const v
                 P.na = d.angles;
                 P.rays = p->det_supersample;
                 P.accumulate = 0;
+                P.gathered = gathered;
                 fp_scale(g->kind, dir, g->vol_scale, force_noncube, p->output_scale, P.f1, P.f2, P.mul);
                 if (dir == 0) { P.n0 = d.vol_x; P.n1 = d.vol_y; P.n2 = d.vol_z; }
                 else if (dir == 1) { P.n0 = d.vol_y; P.n1 = d.vol_x; P.n2 = d.vol_z; }
@@ -470,11 +580,7 @@ b2t_status matched_bp3d_impl(const b2t_geom3d *g, const b2t_params3d *p, const v
                 for (size_t c0 = 0; c0 < views.size() && st == B2T_OK; c0 += FP_MAX_VIEWS) {
                     const size_t cn = std::min(views.size() - c0, (size_t)FP_MAX_VIEWS);
                     P.nviews = (int)cn;
-                    for (size_t i = 0; i < cn; ++i) {
-                        const int a = views[c0 + i];
-                        fp_view_coeffs(g->kind, g->views[a], d, dir, P.views[i]);
-                        P.views[i].a = a;
-                    }
+                    for (size_t i = 0; i < cn; ++i) P.views[i] = coeffs[views[c0 + i]];
                     if (dir == 2) {
                         dim3 grid((unsigned)cn, (d.det_u + 31) / 32, (d.det_v + 7) / 8);
                         if (dtype == B2T_F32) st = launch_T<float>(P, grid, s);
@@ -498,15 +604,15 @@ b2t_status matched_bp3d_impl(const b2t_geom3d *g, const b2t_params3d *p, const v
                             else fp3d_transpose_cols_kernel<__nv_bfloat16, false><<<grid, dim3(32, 8), 0, s>>>(P);
                         }
                         count_launches(1);
-                        g_scatter_launches.fetch_add(1);
+                        if (!gathered) g_scatter_launches.fetch_add(1);
                         if (cudaGetLastError() != cudaSuccess) st = fail(B2T_ERR_CUDA, "matched bp (cells) launch");
                     }
                 }
             }
             delete Lp;
             B2T_TRY(st);
-            const int accumulate = (mode == B2T_MODE_ADD) ? 1 : 0;
-            dim3 grid((d.vol_z + 127) / 128, d.vol_x, d.vol_y);
+            // (fewer blocks where they may have nothing to do)
+            dim3 grid((d.vol_z + 127) / 128, gathered ? (d.vol_x + 7) / 8 : d.vol_x, d.vol_y);
             const float4 *c0 = need[0] && !slab[0] ? cacc[0].as<float4>() : nullptr;
             const float4 *c1 = need[1] && !slab[1] ? cacc[1].as<float4>() : nullptr;
             const float *az = need[2] ? sz.as<float>() : nullptr;
@@ -517,14 +623,14 @@ b2t_status matched_bp3d_impl(const b2t_geom3d *g, const b2t_params3d *p, const v
             matched_slab_dims(d, 1, ay1, mz);
             if (dtype == B2T_F32)
                 fold_cells<float><<<grid, 128, 0, s>>>(c0, c1, az, m0, m1, ay0, ay1, mz, d.vol_x, d.vol_y, d.vol_z,
-                                                       static_cast<float *>(vol), vol_pitch, accumulate);
+                                                       static_cast<float *>(vol), vol_pitch, accumulate, gathered);
             else if (dtype == B2T_F16)
                 fold_cells<__half><<<grid, 128, 0, s>>>(c0, c1, az, m0, m1, ay0, ay1, mz, d.vol_x, d.vol_y,
-                                                        d.vol_z, static_cast<__half *>(vol), vol_pitch, accumulate);
+                                                        d.vol_z, static_cast<__half *>(vol), vol_pitch, accumulate, gathered);
             else
                 fold_cells<__nv_bfloat16><<<grid, 128, 0, s>>>(c0, c1, az, m0, m1, ay0, ay1, mz, d.vol_x, d.vol_y,
                                                                d.vol_z, static_cast<__nv_bfloat16 *>(vol),
-                                                               vol_pitch, accumulate);
+                                                               vol_pitch, accumulate, gathered);
             count_launches(1);
             B2T_CUDA_TRY(cudaGetLastError(), "matched bp fold launch");
             return B2T_OK;
@@ -598,7 +704,6 @@ b2t_status matched_bp3d_impl(const b2t_geom3d *g, const b2t_params3d *p, const v
     delete Lp;
     const float *a = (need[1] || need[2]) ? sa.as<float>() : nullptr;
     const float *b = need[0] ? sb.as<float>() : nullptr;
-    const int accumulate = (mode == B2T_MODE_ADD) ? 1 : 0;
     if (dtype == B2T_F32) return launch_fold<float>(a, b, d, vol, vol_pitch, accumulate, s);
     if (dtype == B2T_F16) return launch_fold<__half>(a, b, d, vol, vol_pitch, accumulate, s);
     return launch_fold<__nv_bfloat16>(a, b, d, vol, vol_pitch, accumulate, s);

@@ -32,11 +32,10 @@
 //
 // Bound by instruction issue (0.77 a cycle and scheduler; a column of 64 voxels
 // takes about 75 instructions, a third of them for its up to four terms).
-// Whole calls, scattered and gathered: 192^3 x 240 views, 288^2 detector 5.7 and
-// 4.8 ms, 256^3 x 360 19.4 and 16.4 ms, 128^3 x 180 1.34 and 1.27 ms (without the
-// test for zero columns 4.5, 15.2 and 1.20 ms).  512^3 x 720 on projections that
-// are mostly zero, whose rays the scatter skips: 261 and 282 ms (the scatter takes
-// 372 ms on dense ones).
+// Whole calls on dense projections, scattered and gathered: 192^3 x 240 views,
+// 288^2 detector 5.36 and 4.59 ms, 256^3 x 360 19.0 and 15.6 ms.  Which calls are
+// gathered is decided by the volume and the scan (matched_gather_eligible) and, on
+// the device, by how many rays hold a value (matched.cu).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -44,8 +43,6 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
-#include <cstdlib>
-#include <string>
 #include <vector>
 
 #include "b2t_internal.h"
@@ -86,6 +83,7 @@ struct MGPrep {
     int *bad;           // [view]: 1 where some weighted value is infinite or NaN (cleared before)
     int nu, nv, na, pitch, half;
     int nviews, first;  // views of this launch, index of its first one in the gather's order
+    const int *run;     // 0 there: the call is scattered (null: gathered)
     float f1[2], f2[2], mul[2];
     float mid[2];       // middle slice of either direction
     signed char dir[MG_MAX_VIEWS];
@@ -101,6 +99,7 @@ struct MGLaunch {
     int nx, ny, nz;
     int nx_views, nviews;  // x-major views come first
     int nzb, splits;
+    const int *run;        // as above
     void *out;             // volume [z][y][x], or FP32 partial sums [split][z][y][x]
     long long out_pitch;
     int accumulate;
@@ -112,41 +111,48 @@ template <> __device__ __forceinline__ float mg_store<float>(float v) { return v
 template <> __device__ __forceinline__ __half mg_store<__half>(float v) { return __float2half_rn(v); }
 template <> __device__ __forceinline__ __nv_bfloat16 mg_store<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
-// Tiles of 32 columns x 32 rows of one view, transposed through shared memory.
+// Tiles of 32 columns x 32 rows of one view, transposed through shared memory; a
+// block takes several (a block that has nothing to do, in a call that is
+// scattered, takes as long to launch as one that has).
+constexpr int PREP_TILES = 6;
 template <typename T> __global__ void __launch_bounds__(256) matched_prep_kernel(const __grid_constant__ MGPrep L)
 {
     __shared__ float tile[32][33];
+    if (L.run && *L.run == 0) return;
     const int i = blockIdx.z;
     const FPView &V = L.views[i];
     const int dir = L.dir[i];
     const long long gi = L.first + i;
-    const int u0 = blockIdx.x * 32, v0 = blockIdx.y * 32;
+    const int u0 = blockIdx.x * 32;
     const int u = u0 + threadIdx.x;
     const float uu = (float)u + 0.5f - 0.5f * (float)L.nu;
     const float den = fmaf(uu, V.e[1], V.e[0]);
     const float inv = 1.0f / den;
     const float A1 = fmaf(uu, V.m1[1], V.m1[0]) * inv;
-    for (int r = threadIdx.y; r < 32; r += 8) {
-        const int v = v0 + r;
-        float y = 0.0f;
-        if (u < L.nu && v < L.nv) {
-            const float vv = (float)v + 0.5f - 0.5f * (float)L.nv;
-            const float A2 = fmaf(vv, V.m2[2], fmaf(uu, V.m2[1], V.m2[0])) * inv;
-            const float sc = sqrtf(fmaf(A1 * A1, L.f1[dir], fmaf(A2 * A2, L.f2[dir], 1.0f))) * L.mul[dir];
-            y = mg_load(static_cast<const T *>(L.proj)[((size_t)v * L.na + V.a) * L.proj_pitch + u]) * sc;
+    for (int v0 = blockIdx.y * 32; v0 < L.pitch; v0 += gridDim.y * 32) {
+        for (int r = threadIdx.y; r < 32; r += 8) {
+            const int v = v0 + r;
+            float y = 0.0f;
+            if (u < L.nu && v < L.nv) {
+                const float vv = (float)v + 0.5f - 0.5f * (float)L.nv;
+                const float A2 = fmaf(vv, V.m2[2], fmaf(uu, V.m2[1], V.m2[0])) * inv;
+                const float sc = sqrtf(fmaf(A1 * A1, L.f1[dir], fmaf(A2 * A2, L.f2[dir], 1.0f))) * L.mul[dir];
+                y = mg_load(static_cast<const T *>(L.proj)[((size_t)v * L.na + V.a) * L.proj_pitch + u]) * sc;
+            }
+            tile[r][threadIdx.x] = y;
         }
-        tile[r][threadIdx.x] = y;
-    }
-    __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += 8) {
-        const int v = v0 + threadIdx.x;
-        const float y = tile[threadIdx.x][r];
-        const bool any = __any_sync(0xffffffffu, y != 0.0f);
-        const bool off = __any_sync(0xffffffffu, !(fabsf(y) <= FLT_MAX));
-        if (u0 + r >= L.nu) continue;
-        if (v < L.pitch) L.rows[(gi * L.nu + u0 + r) * L.pitch + v] = y;
-        if (any && threadIdx.x == 0) L.live[gi * L.nu + u0 + r] = 1;
-        if (off && threadIdx.x == 0) L.bad[gi] = 1;
+        __syncthreads();
+        for (int r = threadIdx.y; r < 32; r += 8) {
+            const int v = v0 + threadIdx.x;
+            const float y = tile[threadIdx.x][r];
+            const bool any = __any_sync(0xffffffffu, y != 0.0f);
+            const bool off = __any_sync(0xffffffffu, !(fabsf(y) <= FLT_MAX));
+            if (u0 + r >= L.nu) continue;
+            if (v < L.pitch) L.rows[(gi * L.nu + u0 + r) * L.pitch + v] = y;
+            if (any && threadIdx.x == 0) L.live[gi * L.nu + u0 + r] = 1;
+            if (off && threadIdx.x == 0) L.bad[gi] = 1;
+        }
+        __syncthreads();
     }
     if (blockIdx.y == 0 && threadIdx.y == 0 && u < L.nu) {
         // rows are counted from `half`, near the detector's centre
@@ -304,6 +310,7 @@ __global__ void __launch_bounds__(32 * T, 1024 / (32 * T)) matched_gather_kernel
 {
     extern __shared__ __align__(16) float sums[];  // [y][x][MG_ZP]
     static_assert(T * T * MG_ZP % 4 == 0, "the columns' float4 are aligned");
+    if (L.run && *L.run == 0) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     MGStep *steps = reinterpret_cast<MGStep *>(sums + T * T * MG_ZP);
     int *texels = reinterpret_cast<int *>(steps + T * 32);
@@ -388,8 +395,9 @@ __global__ void __launch_bounds__(32 * T, 1024 / (32 * T)) matched_gather_kernel
 // out (=|+=) the sum of the partial volumes, in order.
 template <typename T>
 __global__ void matched_fold_splits(const float *__restrict__ part, int splits, int nx, long long rows, T *out,
-                                    long long pitch, int accumulate)
+                                    long long pitch, int accumulate, const int *__restrict__ run)
 {
+    if (run && *run == 0) return;
     const long long n = rows * nx;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         float r = part[i];
@@ -401,18 +409,61 @@ __global__ void matched_fold_splits(const float *__restrict__ part, int splits, 
     }
 }
 
+// Which calls are gathered.  A gather takes time by columns x z of the tiles it
+// launches, whether they hold voxels, have rows or not; a scatter by the samples
+// of the rays there are.  Gathered over scattered time on dense projections
+// (cone, magnification 1.5, 1.2 pixels):
+//  - MG_MIN_SHARE: of the tiles' voxels in all waves of blocks, weighted by the
+//    tile's borders, the share that lies in the volume and before the detector.
+//    192^3 0.89: 0.80 to 0.89; 256^3 and 256^2 x 128 0.87: 0.75 to 0.91; 224^2 x
+//    168 0.87: 0.77 to 0.86; 128^3 0.79: 0.89 to 1.03; 224^3 0.77: 0.87 to 0.98; 192^2 x
+//    144 0.66: 1.04 to 1.15; 160^3 0.51: 1.06 to 1.25; 96^3 0.66: 1.06 to 1.23;
+//    256^3 with 300, 250 and 160 of the 320 rows of its shadow: 0.90, 1.09, 1.62.
+//  - MG_MAX_SPACING of the rows, in texels at the volume's middle: 0.57 0.68, 0.8
+//    0.82, 0.97 0.88, 1.0 0.91, 1.22 1.2.
+//  - MG_MAX_COLUMNS, of the columns, on average over the views (on a full orbit
+//    1.12 times that of a view along an axis): 0.34 0.69, 1.0 0.84, 1.1 0.87, 1.5 0.95,
+//    2.2 1.08 to 1.16.
+//  - MG_MIN_WORK, voxels times views: 192^3 x 60 (4.2e8) 0.80, 128^2 x 64 x 120
+//    (1.3e8) 1.00, 96^3 x 60 (5e7) 1.06.
+constexpr double MG_MIN_SHARE = 0.85;
+constexpr double MG_MAX_SPACING = 1.0;
+constexpr double MG_MAX_COLUMNS = 1.15;
+constexpr double MG_MIN_WORK = 3e8;
+
+// Tiles of 16 x 16 voxels unless the blocks of 8 x 8 ones fill the GPU's
+// slots (two blocks of 16 warps an SM, or four of 8) so much better that it
+// makes up for their wider borders (9 / 8 texels' columns a
+// tile instead of 17 / 16, and the walks' set-up twice as often).
+struct MGTiling {
+    int tile, nzb, splits;
+    double share;  // voxels of the volume to those of all slots' waves
+};
+b2t_status mg_tiling(const b2t_dims3d &d, MGTiling &t)
+{
+    int dev = 0, sms = 0;
+    B2T_CUDA_TRY(cudaGetDevice(&dev), "matched bp device");
+    B2T_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "matched bp SM count");
+    t.nzb = (int)((d.vol_z + MG_Z - 1) / MG_Z);
+    auto blocks = [&](int T) { return (long long)((d.vol_x + T - 1) / T) * ((d.vol_y + T - 1) / T) * t.nzb; };
+    auto cost = [&](int T, long long n) {  // of n blocks
+        const long long slots = (T == 8 ? 4LL : 2LL) * sms;
+        return (double)((n + slots - 1) / slots * slots) * T * T * (T == 8 ? 1.1 : 1.0);
+    };
+    t.tile = cost(8, blocks(8)) < cost(16, blocks(16)) ? 8 : 16;
+    // small volumes: the views split over several blocks a tile, as many as
+    // the slots hold
+    const long long n = blocks(t.tile);
+    t.splits = (int)std::max<long long>(
+        1, std::min<long long>({(t.tile == 8 ? 4LL : 2LL) * sms / n, 8, (long long)d.angles / 8}));
+    t.share = (double)d.vol_x * d.vol_y * d.vol_z * t.splits / (cost(t.tile, n * t.splits) * MG_Z);
+    return B2T_OK;
+}
+
 // The view in FP64 terms of its rounded coefficients: one sign of the
 // denominator over the detector, rows along +z at least 1/4 texel apart at
 // every slice and on average at most MG_MAX_SPACING, and columns that do not
 // turn round between the slices.
-// A gather takes time by columns x z, a scatter by samples, so what decides
-// between them is the rows' spacing in texels.  Scattered and gathered, 256^3 x
-// 360: spacing 0.75 19.4 and 16.4 ms, 0.98 14.4 and 13.0 ms; scattered at 1.22
-// 10.6 ms.
-constexpr double MG_MAX_SPACING = 1.0;
-// Voxels times views from which on views are gathered: 128^3 x 180 (3.8e8) takes
-// 1.34 ms scattered and 1.27 gathered, 96^3 x 120 (1.1e8) 0.45 and 0.46.
-constexpr double MG_MIN_WORK = 3e8;
 bool gather_view_ok(const FPView &w, const b2t_dims3d &d, int dir)
 {
     if (w.e[2] != 0.0f || w.m1[2] != 0.0f || w.n1[2] != 0.0f) return false;
@@ -464,10 +515,10 @@ template <typename S> b2t_status launch_gather(const MGLaunch &L, int tile, cuda
 
 template <typename T>
 b2t_status launch_split_fold(const float *part, int splits, const b2t_dims3d &d, void *vol, size_t pitch, int accumulate,
-                             cudaStream_t s)
+                             const int *run, cudaStream_t s)
 {
     matched_fold_splits<T><<<1184, 256, 0, s>>>(part, splits, (int)d.vol_x, (long long)d.vol_y * d.vol_z,
-                                                static_cast<T *>(vol), (long long)pitch, accumulate);
+                                                static_cast<T *>(vol), (long long)pitch, accumulate, run);
     count_launches(1);
     B2T_CUDA_TRY(cudaGetLastError(), "matched bp (gather) fold launch");
     return B2T_OK;
@@ -475,26 +526,36 @@ b2t_status launch_split_fold(const float *part, int splits, const b2t_dims3d &d,
 
 }  // namespace
 
-bool matched_gather_eligible(const b2t_geom3d *g, const b2t_params3d *p, const std::vector<int> &dirs)
+bool matched_gather_eligible(const b2t_geom3d *g, const b2t_params3d *p, const std::vector<int> &dirs,
+                             const std::vector<FPView> &coeffs, bool pays)
 {
     const b2t_dims3d &d = g->dims;
     if (p->det_supersample != 1 || d.angles == 0) return false;
-    // B2T_MATCHED_PATH=gather: whatever the size (tests)
-    const char *e = std::getenv("B2T_MATCHED_PATH");
-    if ((double)d.vol_x * d.vol_y * d.vol_z * d.angles < MG_MIN_WORK && !(e && std::string(e) == "gather")) return false;
     // positions and row indices are split in FP32 around 1.5 * 2^23
     if (d.vol_x > 32768 || d.vol_y > 32768 || d.vol_z > 32768 || d.det_u > 32768 || d.det_v > 32768) return false;
-    FPView w;
+    MGTiling t{};
+    if (pays) {
+        if ((double)d.vol_x * d.vol_y * d.vol_z * d.angles < MG_MIN_WORK) return false;
+        if (mg_tiling(d, t) != B2T_OK || t.share < MG_MIN_SHARE) return false;
+    }
+    double columns = 0.0;
     for (uint32_t a = 0; a < d.angles; ++a) {
         if (dirs[a] > 1) return false;
-        fp_view_coeffs(g->kind, g->views[a], d, dirs[a], w);
+        const FPView &w = coeffs[a];
         if (!gather_view_ok(w, d, dirs[a])) return false;
+        // the volume's middle: spacing of the rows, of the columns
+        const double mid = 0.5 * ((dirs[a] == 0 ? d.vol_x : d.vol_y) - 1.0);
+        const double rows = (w.m2[2] * mid + w.n2[2]) / w.e[0];
+        const double k1 = w.m1[0] * mid + w.n1[0], k1u = w.m1[1] * mid + w.n1[1];
+        columns += std::abs(k1u * w.e[0] - k1 * w.e[1]) / ((double)w.e[0] * w.e[0]);
+        if (pays && t.share * std::min(1.0, rows * d.det_v / d.vol_z) < MG_MIN_SHARE) return false;
     }
-    return true;
+    return !pays || columns <= MG_MAX_COLUMNS * d.angles;
 }
 
 b2t_status matched_gather(const b2t_geom3d *g, const b2t_params3d *p, const void *proj, size_t proj_pitch, void *vol,
-                          size_t vol_pitch, int32_t dtype, int accumulate, const std::vector<int> &dirs, cudaStream_t s)
+                          size_t vol_pitch, int32_t dtype, int accumulate, const std::vector<int> &dirs,
+                          const std::vector<FPView> &coeffs, const int *run, cudaStream_t s)
 {
     const b2t_dims3d &d = g->dims;
     MGLaunch L{};
@@ -512,20 +573,11 @@ b2t_status matched_gather(const b2t_geom3d *g, const b2t_params3d *p, const void
             if (dirs[a] == dir) order.push_back(a);
         if (dir == 0) L.nx_views = (int)order.size();
     }
-    L.nzb = (L.nz + MG_Z - 1) / MG_Z;
-    // Tiles of 16 x 16 voxels unless the blocks of 8 x 8 ones fill the GPU's
-    // slots (two blocks of 16 warps an SM, or four of 8) so much better that it
-    // makes up for their wider borders (9 / 8 texels' columns a
-    // tile instead of 17 / 16, and the walks' set-up twice as often)
-    auto blocks = [&](int t) { return (long long)((L.nx + t - 1) / t) * ((L.ny + t - 1) / t) * L.nzb; };
-    auto cost = [&](int t, long long slots) {
-        return (double)((blocks(t) + slots - 1) / slots * slots) * t * t * (t == 8 ? 1.1 : 1.0);
-    };
-    const int tile = cost(8, 592) < cost(16, 296) ? 8 : 16;
-    // small volumes: the views split over several blocks a tile, as many as
-    // the slots hold
-    L.splits = (int)std::max<long long>(
-        1, std::min<long long>({(tile == 8 ? 592 : 296) / blocks(tile), 8, (long long)d.angles / 8}));
+    MGTiling t;
+    B2T_TRY(mg_tiling(d, t));
+    const int tile = t.tile;
+    L.nzb = t.nzb;
+    L.splits = t.splits;
     Scratch rows, cols, recs, live, part;
     const size_t ncol = (size_t)d.angles * d.det_u;
     B2T_TRY(rows.alloc(ncol * L.pitch * sizeof(float), s, "matched bp weighted rows"));
@@ -536,6 +588,7 @@ b2t_status matched_gather(const b2t_geom3d *g, const b2t_params3d *p, const void
     B2T_CUDA_TRY(cudaMemsetAsync(live.as<void>(), 0, flags, s), "matched bp live columns");
     const size_t vox = (size_t)d.vol_x * d.vol_y * d.vol_z;
     if (L.splits > 1) B2T_TRY(part.alloc(L.splits * vox * sizeof(float), s, "matched bp partial volumes"));
+    L.run = run;
     L.rows = rows.as<float>();
     L.cols = cols.as<MGColumn>();
     L.recs = recs.as<MGRecord>();
@@ -546,6 +599,7 @@ b2t_status matched_gather(const b2t_geom3d *g, const b2t_params3d *p, const void
         MGPrep &P = *Pp;
         P.proj = proj;
         P.proj_pitch = (long long)proj_pitch;
+        P.run = run;
         P.rows = rows.as<float>();
         P.cols = cols.as<MGColumn>();
         P.recs = recs.as<MGRecord>();
@@ -566,11 +620,10 @@ b2t_status matched_gather(const b2t_geom3d *g, const b2t_params3d *p, const void
             P.nviews = (int)std::min(order.size() - c0, (size_t)MG_MAX_VIEWS);
             for (int i = 0; i < P.nviews; ++i) {
                 const uint32_t a = order[c0 + i];
-                fp_view_coeffs(g->kind, g->views[a], d, dirs[a], P.views[i]);
-                P.views[i].a = (int)a;
+                P.views[i] = coeffs[a];
                 P.dir[i] = (signed char)dirs[a];
             }
-            const dim3 grid((L.nu + 31) / 32, (L.pitch + 31) / 32, P.nviews);
+            const dim3 grid((L.nu + 31) / 32, (L.pitch + 32 * PREP_TILES - 1) / (32 * PREP_TILES), P.nviews);
             if (dtype == B2T_F32) st = launch_prep<float>(P, grid, s);
             else if (dtype == B2T_F16) st = launch_prep<__half>(P, grid, s);
             else st = launch_prep<__nv_bfloat16>(P, grid, s);
@@ -583,9 +636,9 @@ b2t_status matched_gather(const b2t_geom3d *g, const b2t_params3d *p, const void
         L.out_pitch = L.nx;
         L.accumulate = 0;
         B2T_TRY(launch_gather<float>(L, tile, s));
-        if (dtype == B2T_F32) return launch_split_fold<float>(part.as<float>(), L.splits, d, vol, vol_pitch, accumulate, s);
-        if (dtype == B2T_F16) return launch_split_fold<__half>(part.as<float>(), L.splits, d, vol, vol_pitch, accumulate, s);
-        return launch_split_fold<__nv_bfloat16>(part.as<float>(), L.splits, d, vol, vol_pitch, accumulate, s);
+        if (dtype == B2T_F32) return launch_split_fold<float>(part.as<float>(), L.splits, d, vol, vol_pitch, accumulate, run, s);
+        if (dtype == B2T_F16) return launch_split_fold<__half>(part.as<float>(), L.splits, d, vol, vol_pitch, accumulate, run, s);
+        return launch_split_fold<__nv_bfloat16>(part.as<float>(), L.splits, d, vol, vol_pitch, accumulate, run, s);
     }
     L.out = vol;
     L.out_pitch = (long long)vol_pitch;

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <memory>
+#include <string>
 #include <vector>
 
 #include "b2tomo.h"
@@ -38,6 +39,7 @@ struct FPLaunch {
     int accumulate;         // 1: proj += result, 0: proj = result
     float f1, f2, mul;      // ray length factors and output scale
     int nviews;
+    const int *gathered = nullptr;  // matched BP: set where the gather runs instead (null: this runs)
     FPView views[FP_MAX_VIEWS];
 };
 
@@ -175,8 +177,8 @@ size_t matched_slab_acc_bytes(const b2t_dims3d &d, int dir);
 b2t_status matched_slab_scatter(const b2t_geom3d *g, const b2t_params3d *p, const void *proj, size_t proj_pitch,
                                 int32_t dtype, int dir, const std::vector<int> &dirs, float *acc, cudaStream_t s);
 b2t_status matched_path_stats_impl(uint64_t *stats);
-// launches of matched.cu's scatter kernels since the last call
-unsigned long long matched_scatter_launches_take();
+// launches of matched.cu's scatter kernels that did their work since the last call
+b2t_status matched_scatter_launches_take(unsigned long long *n);
 // proj (=|+=) FP of the volume the cells hold, for the views of g (same
 // volume dimensions as at build time; every view's marching axis built).
 b2t_status fp3d_cells_project(const b2t_geom3d *g, const b2t_params3d *p, const FPCells &c, void *proj,
@@ -207,10 +209,17 @@ b2t_status bp3d_impl(const b2t_geom3d *g, const b2t_params3d *p, const void *pro
 // use the pair layout (padded_elem_size).
 bool bp_pairs(int32_t dtype, const b2t_params3d *p);
 size_t padded_proj_bytes(const b2t_dims3d &d, int32_t dtype, bool pairs);
-// matched BP gathered per voxel: whether every view allows it, and the call
-bool matched_gather_eligible(const b2t_geom3d *g, const b2t_params3d *p, const std::vector<int> &dirs);
+// matched BP gathered per voxel: whether every view allows it (pays: and it is
+// faster than the scatter on projections without zeros), and the call.  run: the
+// call's kernels return at once where *run is 0 (null: they run).
+// coeffs: the views' coefficients along their directions, .a their indices.
+bool matched_gather_eligible(const b2t_geom3d *g, const b2t_params3d *p, const std::vector<int> &dirs,
+                             const std::vector<FPView> &coeffs, bool pays);
 b2t_status matched_gather(const b2t_geom3d *g, const b2t_params3d *p, const void *proj, size_t proj_pitch, void *vol,
-                          size_t vol_pitch, int32_t dtype, int accumulate, const std::vector<int> &dirs, cudaStream_t s);
+                          size_t vol_pitch, int32_t dtype, int accumulate, const std::vector<int> &dirs,
+                          const std::vector<FPView> &coeffs, const int *run, cudaStream_t s);
+// B2T_MATCHED_PATH (tests): gather, scatter or slab; empty when not set
+std::string matched_path_env();
 // The zero-padded projection buffer of projections proj (row pitch in
 // texels) in the layout bp_pairs selects.
 b2t_status pad_projections_impl(const void *proj, size_t pitch, const b2t_dims3d &d, void *padded, int32_t dtype,

@@ -87,8 +87,10 @@ b2t_status b2t_fp_path_stats(uint64_t stats[4]);
  * backprojection since the last call: stats[0] slices whose accumulation box
  * CTAs of the slab transpose kept in shared memory, stats[1] slices they
  * scattered straight into global memory (a box too large for a slice
- * buffer), stats[2] slab transpose launches, stats[3] launches of the
- * per-sample scatter kernels (views the slab transpose does not take).
+ * buffer), stats[2] slab transpose launches (B2T_MATCHED_PATH=slab only),
+ * stats[3] launches of the per-sample scatter kernels.  A call that leaves
+ * all four zero was gathered per voxel; a call that chooses on the device
+ * between gather and scatter counts its scatter launches when it scattered.
  * Synchronises the device.  A performance diagnostic; the reference has no
  * counterpart. */
 b2t_status b2t_matched_path_stats(uint64_t stats[4]);

@@ -115,12 +115,18 @@ def test_scattered_views(astra, orc, case, monkeypatch):
     _check(astra, orc, pg, vg, monkeypatch, gathered=False)
 
 
+# volumes whose tiles fill the GPU's slots well (16 x 16 blocks and 8 x 8 ones)
+FULL = ((256, 256, 128, 60), (192, 192, 192, 60))
+
+
 def test_default_size(astra, orc):
-    """Above 3e8 voxel views the gather is the default, both blocks' shapes and
-    split views among them, and needs no scatter."""
-    for n, na in ((64, 1200), (128, 150)):
-        vg = astra.create_vol_geom(n, n, n)
-        pg = astra.create_proj_geom('cone', 1.0, 1.0, n, n, np.linspace(0, 2 * np.pi, na, endpoint=False), 4.0 * n, n)
+    """Where the tiles fill the GPU, dense projections are gathered and need no
+    scatter."""
+    for nx, ny, nz, na in FULL:
+        n = nx
+        vg = astra.create_vol_geom(ny, nx, nz)
+        pg = astra.create_proj_geom('cone', 1.0, 1.0, nz + nz // 4, n + n // 4, np.linspace(0, 2 * np.pi, na, endpoint=False),
+                                    4.0 * n, n)
         pr = astra.Projector3D(pg, vg, {'ProjectionKernel': 'matched_bp'})
         x = torch.randn(pr.vol_shape, device='cuda')
         y = torch.rand(pr.proj_shape, device='cuda')
@@ -167,3 +173,76 @@ def test_non_finite_values(astra, orc, pv, dtype, value, monkeypatch):
         assert not np.isfinite(got[met]).any(), path
         assert np.isfinite(got[missed]).all(), path
         assert rel_l2(got[missed], ref[missed]) < {"float32": 1e-5, "float16": 1e-3}[dtype]
+
+
+def _default(astra, vol, na, du, dv, px=1.0, so=4.0, od=1.0):
+    nx, ny, nz = vol
+    pg = astra.create_proj_geom('cone', px, px, dv, du, np.linspace(0, 2 * np.pi, na, endpoint=False), so * nx, od * nx)
+    return astra.Projector3D(pg, astra.create_vol_geom(ny, nx, nz), {'ProjectionKernel': 'matched_bp'})
+
+
+@pytest.mark.parametrize("vol,na,du,dv,px", [
+    ((64, 64, 64), 1200, 80, 80, 1.0),      # blocks that do not fill the slots
+    ((192, 192, 130), 100, 240, 170, 1.0),  # tiles past the volume's last slice
+    ((256, 256, 128), 60, 320, 80, 1.0),    # rows for part of the volume
+    ((256, 256, 128), 60, 100, 60, 3.0),    # columns and rows far apart
+    ((192, 192, 192), 20, 240, 240, 1.0),   # little work
+])
+def test_default_scatters_where_the_gather_is_slower(astra, vol, na, du, dv, px):
+    pr = _default(astra, vol, na, du, dv, px)
+    y, x = torch.rand(pr.proj_shape, device='cuda'), torch.zeros(pr.vol_shape, device='cuda')
+    _scatters()
+    pr.bp(y, x)
+    assert _scatters() > 0
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("keep", [0.0, 0.5, 0.87, 0.93, 1.0])
+def test_choice_by_the_share_of_values(astra, keep, mode, dtype, monkeypatch):
+    """Projections with a value on nine rays in ten or more are gathered, others
+    scattered, with the values of the other choice."""
+    pr = _default(astra, FULL[1][:3], FULL[1][3], 240, 240)
+    t = getattr(torch, dtype)
+    gen = torch.Generator('cuda').manual_seed(int(100 * keep))
+    y = torch.rand(pr.proj_shape, device='cuda', generator=gen) + 0.5
+    y = (y * (torch.rand(pr.proj_shape, device='cuda', generator=gen) < keep)).to(t)
+    base = torch.rand(pr.vol_shape, device='cuda', generator=gen).to(t)
+    out = {}
+    for path in (None, "gather", "scatter"):
+        if path:
+            monkeypatch.setenv("B2T_MATCHED_PATH", path)
+        out[path] = base.clone()
+        _scatters()
+        pr.bp(y, out[path], mode=mode)
+        n = _scatters()
+        assert (n == 0) == (keep > 0.9 if path is None else path == "gather")
+    monkeypatch.delenv("B2T_MATCHED_PATH")
+    a, b, c = (out[k].double() for k in (None, "gather", "scatter"))
+    # the scatter's order differs from call to call by 1e-7, which one value in two
+    # thousand (FP16) rounds apart, by 2^-10
+    again = {"float32": 1e-6, "float16": 1e-4, "bfloat16": 1e-3}[dtype]
+    assert torch.equal(a, b) if keep > 0.9 else float((a - c).norm()) <= again * float(c.norm())
+    # FP32 sums in another order, and one rounding of the output
+    tol = {"float32": 1e-5, "float16": 1e-3, "bfloat16": 8e-3}[dtype]
+    assert float((b - c).norm()) <= tol * float(c.norm())
+
+
+def test_choice_is_made_at_each_replay(astra):
+    """A captured call holds both ways and chooses by the projections of the replay."""
+    pr = _default(astra, FULL[1][:3], FULL[1][3], 240, 240)
+    y, x = torch.rand(pr.proj_shape, device='cuda') + 0.5, torch.zeros(pr.vol_shape, device='cuda')
+    pr.bp(y, x)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        pr.bp(y, x)
+    for keep in (1.0, 0.3, 1.0):
+        y.copy_((torch.rand_like(y) + 0.5) * (torch.rand_like(y) < keep))
+        want = pr.bp(y, torch.zeros_like(x))
+        x.fill_(-3.0)
+        _scatters()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert (_scatters() == 0) == (keep == 1.0)
+        assert float((x - want).norm()) <= 1e-6 * float(want.norm())
