@@ -135,6 +135,7 @@ SIGNATURES = {
     "b2t_set_device": (_I32, [_I32]),
     "b2t_device_errors": (_I32, [_P]),
     "b2t_bp_path_stats": (_I32, [_P]),
+    "b2t_bp_packed_columns": (_I32, [_P]),
     "b2t_fp_path_stats": (_I32, [_P]),
     "b2t_matched_path_stats": (_I32, [_P]),
     "b2t_cone_views": (_I32, [_U32, _U32, _U32, _F, _F, _F, _F, _P, _P]),

@@ -172,6 +172,14 @@ b2t_status b2t_bp_path_stats(uint64_t *stats)
     return bp_path_stats_impl(stats);
 }
 
+b2t_status b2t_bp_packed_columns(uint64_t *columns)
+{
+    clear_error();
+    if (!columns) return fail(B2T_ERR_INVALID_ARG, "b2t_bp_packed_columns: null pointer");
+    B2T_CUDA_TRY(cudaDeviceSynchronize(), "b2t_bp_packed_columns synchronize");
+    return bp_packed_columns_impl(columns);
+}
+
 b2t_status b2t_fp3d(const b2t_geom3d *geom, const b2t_params3d *params, const void *vol, size_t vol_pitch,
                     void *proj, size_t proj_pitch, int32_t dtype, int32_t mode, void *stream)
 {

@@ -60,8 +60,9 @@ static __device__ unsigned int g_b2t_device_errors = 0;
 // shared-memory tile), [1] the general path (other orbits, columns whose
 // rows leave the tile, views read from global memory), [2] lanes idle
 // because their column lies outside the volume; [3] SM cycles the compute
-// warps spent in their view loops, summed over warps.
-static __device__ unsigned long long g_bp_path_stats[4] = {0, 0, 0, 0};
+// warps spent in their view loops, summed over warps; [4] (read by
+// b2t_bp_packed_columns) those of [1] on the packed path of other orbits.
+static __device__ unsigned long long g_bp_path_stats[5] = {0, 0, 0, 0, 0};
 
 namespace {
 
@@ -644,7 +645,7 @@ __global__ void __launch_bounds__(288, BPT_CTAS_PER_SM) bp3d_tma_kernel(const __
                 done = true;
             }
         }
-        if (CIRC && done) ++n_fast;
+        if (done) ++n_fast;
         else if (active) ++n_general;
         else ++n_idle;
         if (active && !done) {
@@ -756,8 +757,8 @@ __global__ void __launch_bounds__(288, BPT_CTAS_PER_SM) bp3d_tma_kernel(const __
     const unsigned w_general = __reduce_add_sync(0xffffffffu, (unsigned)n_general);
     const unsigned w_idle = __reduce_add_sync(0xffffffffu, (unsigned)n_idle);
     if (lane == 0) {
-        atomicAdd(&g_bp_path_stats[0], (unsigned long long)w_fast);
-        atomicAdd(&g_bp_path_stats[1], (unsigned long long)w_general);
+        atomicAdd(&g_bp_path_stats[CIRC ? 0 : 4], (unsigned long long)w_fast);
+        atomicAdd(&g_bp_path_stats[1], (unsigned long long)(CIRC ? w_general : w_general + w_fast));
         atomicAdd(&g_bp_path_stats[2], (unsigned long long)w_idle);
         atomicAdd(&g_bp_path_stats[3], (unsigned long long)(clock64() - t_loop));
     }
@@ -1011,6 +1012,17 @@ b2t_status bp_path_stats_impl(uint64_t *stats)
     const unsigned long long zero[4] = {0, 0, 0, 0};
     B2T_CUDA_TRY(cudaMemcpyToSymbol(g_bp_path_stats, zero, sizeof(zero)), "clear BP path statistics");
     for (int k = 0; k < 4; ++k) stats[k] = v[k];
+    return B2T_OK;
+}
+
+b2t_status bp_packed_columns_impl(uint64_t *columns)
+{
+    unsigned long long v = 0;
+    const size_t at = 4 * sizeof(v);
+    B2T_CUDA_TRY(cudaMemcpyFromSymbol(&v, g_bp_path_stats, sizeof(v), at), "read BP path statistics");
+    const unsigned long long zero = 0;
+    B2T_CUDA_TRY(cudaMemcpyToSymbol(g_bp_path_stats, &zero, sizeof(zero), at), "clear BP path statistics");
+    *columns = v;
     return B2T_OK;
 }
 

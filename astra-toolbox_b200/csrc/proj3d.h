@@ -111,6 +111,7 @@ b2t_status bp3d_tma(const b2t_geom3d *g, int ker, float out_scale, const void *p
                     size_t vol_pitch, int32_t dtype, int32_t mode, cudaStream_t s);
 b2t_status device_errors_impl(uint32_t *flags);
 b2t_status bp_path_stats_impl(uint64_t *stats);
+b2t_status bp_packed_columns_impl(uint64_t *columns);
 b2t_status bp3d_autotune_impl(const b2t_geom3d *g, const b2t_params3d *p, const void *proj, size_t proj_pitch,
                               void *vol, size_t vol_pitch, int32_t dtype, cudaStream_t s, int32_t *vpt_out);
 // One warp waits, bounded by limit cycles, for an mbarrier phase (which 0) or

@@ -65,16 +65,21 @@ b2t_status b2t_set_device(int32_t device);
 b2t_status b2t_device_errors(uint32_t *flags);
 /* Read and clear, for the current device, the path statistics of the
  * TMA-staged cone/parallel backprojection since the last call.  Counts are in
- * voxel-column views (one thread's column of 32 voxels for one view):
+ * voxel-column views (one thread's column of 32 or 16 voxels for one view):
  * stats[0] took the circular-orbit fast path (detector u fixed along the
  * column, every sample from the shared-memory tile of the view's footprint);
- * stats[1] took the general path (non-circular orbits, columns whose rows
+ * stats[1] took another path (non-circular orbits, columns whose rows
  * leave the tile, views whose footprint does not fit a tile and read global
  * memory); stats[2] were idle lanes (columns outside the volume).  stats[3]
  * is the SM cycles the compute warps spent in their view loops, summed over
  * warps.  Synchronises the device.  A performance diagnostic; the reference
  * has no counterpart. */
 b2t_status b2t_bp_path_stats(uint64_t stats[4]);
+/* Read and clear, likewise, how many of the columns in stats[1] took the packed
+ * path of non-circular orbits (u, v and the weight of two voxels at a time,
+ * every sample from the shared-memory tile); the others of such an orbit
+ * went sample by sample. */
+b2t_status b2t_bp_packed_columns(uint64_t *columns);
 /* Read and clear the path statistics of the cone/parallel forward projection
  * since the last call: stats[0] slices that CTAs of the TMA-staged slab
  * kernel read from shared memory, stats[1] slices they read from the slab

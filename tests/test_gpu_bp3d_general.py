@@ -3,6 +3,9 @@ voxel column in every respect (tilted detectors, inclined parallel rays),
 against the direct-load kernel and the FP64 oracle: columns at the ends of
 16- and 32-voxel blocks, small and strong tilts (strong ones leave the tile
 and take the per-sample checks), every storage type."""
+import ctypes
+import importlib
+
 import numpy as np
 import pytest
 
@@ -10,6 +13,15 @@ from conftest import rel_l2
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
+
+
+def _paths():
+    """Voxel-column views on the circular path, on others, and of those on the
+    packed path, since the last call."""
+    lib = importlib.import_module("astra-toolbox_b200._lib").load()
+    st, packed = (ctypes.c_uint64 * 4)(), ctypes.c_uint64(0)
+    assert lib.b2t_bp_path_stats(st) == 0 and lib.b2t_bp_packed_columns(ctypes.byref(packed)) == 0
+    return st[0], st[1], packed.value
 
 
 def _vectors(kind, n, tilt_deg, seed):
@@ -47,7 +59,14 @@ def test_general_orbits(astra, orc, kind, tilt, shape, monkeypatch):
         got = {}
         for dtype in (torch.float32, torch.float16, torch.bfloat16):
             a = torch.zeros(pr.vol_shape, device='cuda', dtype=dtype)
+            _paths()
             pr.bp(tp.to(dtype), a)
+            circular, other, packed = _paths()
+            assert circular == 0 and other > 0
+            if shape == (64, 40, 70):  # (smaller ones cut the columns short of a block)
+                share = packed / other
+                # (no parallel view of these leaves its tile)
+                assert share > 0.99 if tilt == 0.1 or kind == 'parallel3d_vec' else 0.5 < share if tilt == 4.0 else 0.0 < share < 1.0, share
             got[dtype] = a.float().cpu().numpy()
         monkeypatch.setenv("B2T_SIMPLE_BP", "1")
         for dtype, tol in ((torch.float32, 4e-6), (torch.float16, 5e-4), (torch.bfloat16, 4e-3)):
