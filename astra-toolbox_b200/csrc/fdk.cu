@@ -102,7 +102,7 @@ __device__ __forceinline__ float fdk_weight(const FDKWeights &P, int u, int nu, 
 // dst (in-place filtering).
 //
 // The near part is bound by instruction issue (32 taps an output), the rest by
-// memory (read 4, write 4 + 12 bytes a value).  Warps take chunks of 256
+// memory (read 4, write 4 + 6 bytes a value).  Warps take chunks of 256
 // outputs of any of the CTA's rows, 8 consecutive outputs a lane in packed
 // f32x2 (the sliding windows move by one pair a tap, so pairs stay pairs), and
 // pass them through a warp's staging row so that stores are contiguous.

@@ -82,7 +82,7 @@ constexpr int SLAB_THREADS = 32 * (SLAB_WARPS + 1);
 // Slice buffers: four of 3584 z-pairs (28 KB) in the 113 KB that two CTAs per
 // SM leave each, as two stages of two slices.  One wait and one release per two
 // slices take about twelve instructions a slice off the warps (of about 150);
-// measured at 512^3 x 720 / 256^3 x 360 (832^2 / 416^2 detectors): three
+// measured at 512^3 x 720 / 256^3 x 360 (832^2 / 416^2 detectors of 1.2 pixels): three
 // stages of one slice (24 x 160 pairs) 116.9 / 8.84 ms, four stages of one
 // slice 110.2 / 8.52, two stages of two 105.4 / 7.79 and with box widths 128
 // and 176 (wide boxes of rows far from the source fit: 0.7 % of the slices

@@ -265,9 +265,8 @@ __device__ __forceinline__ void sum_part(const LineRay (&ray)[2], bool mixed, in
 // group's FP2D_PARTS ranges of slices one warp each: four times the warps of
 // one per group, which a small problem needs (128^2 x 180 parallel: 33 us with
 // one warp, 24 with two, 18 with four) and a large one does not lose by
-// (1024^2 x 1440: 0.89, 0.97, 0.84 ms).  About ten instructions per sample at
-// half the issue rate: bound by the latency of the loads that miss L1 (one
-// load in eight).
+// (1024^2 x 1440: 0.89, 0.97, 0.84 ms).  Bound by the latency of L2: 44 % of the
+// issue rate, seven sectors in ten miss L1.
 template <int KIND, int CAP>
 __global__ void __launch_bounds__(LINES_THREADS) fp2d_lines_kernel(const __grid_constant__ FP2DLinesLaunch<CAP> L)
 {
@@ -416,9 +415,10 @@ __device__ __forceinline__ void bp_positions(const float *c, const uint64_t (&x2
 // its BP2D_PARTS / WS ranges of views over WS warps.  The CTA stages, ROWS
 // views at a time (ROWS / WS of each of the WS ranges), the window of pairs
 // that its pixels sample, zeros outside the detector, into one of two
-// buffers.  Bound by instruction issue (77 %) with the shared-memory data
-// pipe at 58 %: 1024^2 x 1440 takes 0.62 ms parallel and 0.94 ms fan; reading
-// bordered pairs of the sinogram through L1 instead took 0.84 and 1.56 ms.
+// buffers.  Parallel views are bound by the shared-memory data pipe (78 %, issue
+// 72 %), fan views by instruction issue (69 %, data pipe 56 %): 1024^2 x 1440 takes
+// 0.62 ms parallel and 0.94 ms fan; reading bordered pairs of the sinogram
+// through L1 instead took 0.84 and 1.56 ms.
 template <int KIND, int PX, int WS, int ROWS, int CAP>
 __global__ void __launch_bounds__(LINES_THREADS) bp2d_lines_kernel(const __grid_constant__ BP2DLinesLaunch<CAP> L)
 {

@@ -30,7 +30,7 @@
 //   no two warps share an accumulator, so there are no atomics and the result
 //   does not depend on the order of the blocks.
 //
-// Bound by instruction issue (0.77 a cycle and scheduler; a column of 64 voxels
+// Bound by instruction issue (0.75 a cycle and scheduler; a column of 64 voxels
 // takes about 75 instructions, a third of them for its up to four terms).
 // Whole calls on dense projections, scattered and gathered: 192^3 x 240 views,
 // 288^2 detector 5.36 and 4.59 ms, 256^3 x 360 19.0 and 15.6 ms.  Which calls are

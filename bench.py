@@ -967,8 +967,8 @@ def run_extra(args):
     autograd backward) on the cone workload; one step = one matched BP of the
     phantom's projections; metric GUPS (Nx Ny Nz Nangles / time), with the
     dot-product test <A x, y> = <x, A^T y> (FP64 sums) of this run's output
-    and the path statistics (B2T_MATCHED_PATH=slab selects the slab
-    transpose)."""
+    and the path that ran, with its statistics (B2T_MATCHED_PATH=slab
+    selects the slab transpose, =gather and =scatter the others)."""
     import torch
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
@@ -1086,7 +1086,7 @@ def run_extra(args):
         ups = float(np.prod(pr.vol_shape)) * pr.proj_shape[1]
         value, unit, hib = ups / (ms * 1e-3) / 1e9, "GUPS", True
         metric = "matched BP (exact FP transpose) GUPS at %d^3x%d" % (args.n, args.views)
-        path = "slab" if os.environ.get("B2T_MATCHED_PATH") == "slab" else "scatter"
+        path = "slab" if st[2] else "scatter" if st[3] else "gather"
         extra = {"path": path, "dot_test_rel": abs(lhs - rhs) / abs(lhs),
                  "path_stats": {"slices_in_smem": int(st[0]), "slices_global": int(st[1]),
                                 "slab_launches": int(st[2]), "scatter_launches": int(st[3])}}
@@ -1403,14 +1403,14 @@ def main():
     achieved = alg_bytes / (dom_ms * 1e-3) / 1e9
     # DRAM bytes (read + write) of the dominant call's launches, per call.
     # FP: the bytes per sample of one ncu capture of the FP kernel at 384^3 x
-    # 360 views, 624^2 (21.43 GB for 744.6 M warp-samples of 32 rays; profiles/
-    # cone_fp_slab_384cube_360views.md) times this call's samples; BP: one
+    # 360 views, 624^2 (20.13 GB for 744.6 M warp-samples of 32 rays; profiles/
+    # line_gather_slab_kernels.md) times this call's samples; BP: one
     # capture of this exact workload (profiles/dram_traffic_cone_fpbp_512cube_
     # 720views.md).  Null for other workloads and storage types.
     traffic, traffic_src = None, None
     if (args.n, args.views, args.det, args.dtype) == (N_VOX, N_ANG, N_DET, "float32"):
         if dom == "fp":
-            traffic = (20.96 + 0.47) * 1e9 / (744633280.0 * 32) * units
+            traffic = (19.61 + 0.52) * 1e9 / (744633280.0 * 32) * units
             traffic_src = "scaled by samples from an ncu capture of the FP at 384^3 x 360 views, 624^2"
         else:
             traffic = (15.87 + 0.53 + 0.95 + 0.50) * 1e9
@@ -1423,7 +1423,7 @@ def main():
                 "traffic": traffic, "units_per_launch": units, "bytes_per_unit": 4 * esz,
                 "traffic_note": "DRAM bytes of one whole call (the FP's x- and y-major launches, or the BP's "
                                 "launch), %s; the slice boxes / tiles are re-read on chip, DRAM moves about "
-                                "1/18 of the algorithmic bytes" % traffic_src,
+                                "1/19 of the algorithmic bytes" % traffic_src,
                 "peak_source": "measured on this GPU by b2t_onchip_peak (16-byte streaming loads); the FP "
                                "reads its samples from TMA-staged shared memory, whose measured roof is "
                                "within 1 % of the L1 one",

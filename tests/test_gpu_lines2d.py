@@ -43,6 +43,9 @@ SHAPES = [
     ('fanflat', 900, 850, 30, 1301), ('fanflat', 80, 80, 1100, 25), ('fanflat_vec', 50, 61, 77, 150),
     # detectors so fine that a tile's footprint exceeds the staged window
     ('parallel_fine', 40, 44, 50, 900), ('fanflat_fine', 40, 44, 50, 900),
+    # small images of more than 64 views, whose projections go through lines as well
+    ('parallel', 1, 1, 70, 1), ('parallel', 3, 2, 65, 7), ('parallel', 32, 32, 69, 64), ('parallel', 33, 31, 77, 65),
+    ('fanflat', 1, 1, 66, 3), ('fanflat', 64, 64, 65, 96), ('parallel_fine', 40, 44, 70, 900), ('fanflat_fine', 40, 44, 70, 900),
 ]
 
 
