@@ -17,9 +17,9 @@
 //     (v[z], v[z + 1] - v[z]) in FP32 (z contiguous, a zero border of two texels), so
 //     a bilinear sample is two 8-byte loads and two FMAs along z;
 //   - a CTA traces SLAB_W consecutive views x SLAB_U consecutive detector
-//     columns x up to SLAB_ROWS detector rows (blocks of equal height); a
-//     compute warp owns one column, each lane SLAB_R rows of it (v, v + 32, ...) in both views, so the in-plane
-//     position, texel split and buffer row of a slice are computed once per
+//     columns x up to SLAB_ROWS detector rows (slab_rows); a compute warp owns
+//     one column, each lane SLAB_R rows of it (v, v + 32, ...) in both views, so the
+//     in-plane position, texel split and buffer row of a slice are computed once per
 //     view for SLAB_R rays and the slice's wait and release once for all
 //     SLAB_W x SLAB_R of them;
 //   - a producer warp works out the buffer box of 32 slices at a time (one
@@ -111,11 +111,59 @@ __host__ __device__ constexpr bool slab_fits(int ny, int nz)
            ((ny + SLAB_BOX_Y - 1) / SLAB_BOX_Y) * SLAB_BOX_Y * (nz <= SLAB_WA ? SLAB_WA : SLAB_WB) <= SLAB_SLOT;
 }
 
-// Detector rows of a CTA: the fewest row blocks, of equal height.
-int slab_rows(const b2t_dims3d &d)
+// CTAs of a launch over the slots of the GPU (two an SM).
+double slab_waves(const b2t_dims3d &d, size_t views, int rows)
 {
-    const int blocks = (int)((d.det_v + SLAB_ROWS - 1) / SLAB_ROWS);
-    return 32 * (((int)d.det_v + 32 * blocks - 1) / (32 * blocks));
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) {
+        (void)cudaGetLastError();
+        sms = 148;
+    }
+    const double ctas = (double)((views + SLAB_W - 1) / SLAB_W) * ((d.det_u + SLAB_U - 1) / SLAB_U) *
+                        ((d.det_v + (unsigned)rows - 1) / (unsigned)rows);
+    return ctas / (2 * sms);
+}
+
+// Detector rows of a CTA: the fewest row blocks, of equal height, or full ones and
+// a rest where these have less to do in the volume's shadow (a block works at the
+// slices whose rows it sees; a slice costs it about as much as SLAB_FIXED rows a
+// lane, and their number).  Full and equal blocks, cone, 1.5 times magnified: 256^3
+// x 360 views, 358 rows, share of the work 0.83, 5.87 and 6.71 ms; 200 x 200 x nz, 200
+// views: 165 rows of nz = 122 0.82, 1.31 and 1.46; 330 of 245 0.88, 2.22 and 2.38; 500 of
+// 372 0.92, 3.16 and 3.30; 350 of 293 0.95, 2.39 and 2.37; 180 of 133 0.96, 1.52 and 1.48;
+// 380 of 353 1, 2.72 and 2.50.  In launches of less than SLAB_FULL_WAVES higher blocks
+// take longer where they win in larger ones: 128 x 128 x 245, 330 rows, 4 views 439 and
+// 331 us, 16 (0.7 waves) 301 and 270, 60 (2.7) 524 and 494, 80 (3.6) 502 and 530.
+constexpr double SLAB_FULL_WAVES = 2.8, SLAB_FULL_SHARE = 0.93;
+constexpr int SLAB_FIXED = 5, SLAB_FULL_SLICES = 16;
+template <typename Views> int slab_rows(const b2t_geom3d *g, int dir, const Views &views)
+{
+    const b2t_dims3d &d = g->dims;
+    const int nv = (int)d.det_v, blocks = (nv + SLAB_ROWS - 1) / SLAB_ROWS;
+    const int equal = 32 * ((nv + 32 * blocks - 1) / (32 * blocks));
+    if (equal == SLAB_ROWS || blocks == 1 || slab_waves(d, views.size(), equal) < SLAB_FULL_WAVES) return equal;
+    FPView w;
+    const uint32_t a = (uint32_t)views[views.size() / 2];
+    fp_view_coeffs(g->kind, g->views[a], d, dir, w);
+    int work[2] = {0, 0};  // of full and equal blocks
+    for (int j = 0; j <= SLAB_FULL_SLICES; ++j) {
+        // rows of the shadow, a texel wider than it is, on the middle column of one view
+        const double s = ((dir == 0 ? d.vol_x : d.vol_y) - 1.0) * j / SLAB_FULL_SLICES;
+        const double at = w.m2[0] * s + w.n2[0], step = w.m2[2] * s + w.n2[2];  // (z texels of a row) x e[0]
+        double v[2];
+        for (int k = 0; k < 2; ++k) {
+            v[k] = ((k ? d.vol_z + 1.0 : -2.0) * w.e[0] - at) / step - 0.5 + 0.5 * nv;
+            if (!(std::abs(v[k]) < 1e9)) return equal;
+        }
+        const double lo = std::min(v[0], v[1]), hi = std::max(v[0], v[1]);
+        for (int k = 0; k < 2; ++k) {
+            const int rows = k ? equal : SLAB_ROWS;
+            for (int r = 0; r < nv; r += rows)
+                if (hi >= r && lo < r + rows) work[k] += SLAB_FIXED + (std::min(rows, nv - r) + 31) / 32;
+        }
+    }
+    return work[0] < SLAB_FULL_SHARE * work[1] ? SLAB_ROWS : equal;
 }
 
 // The launch record of the FP and of its transpose (bp3d_slab_matched_kernel,
@@ -1182,20 +1230,15 @@ bool fp_slab_pays(const b2t_geom3d *g, int dir, const std::vector<int> &dirs)
 {
     if (slab_path('s')) return true;
     const b2t_dims3d &d = g->dims;
-    const int rows = slab_rows(d);
-    if (rows < PAY_ROWS) return false;
     std::vector<uint32_t> views;
     for (uint32_t a = 0; a < d.angles; ++a)
         if (dirs[a] == dir) views.push_back(a);
+    if (views.empty()) return true;
+    const int rows = slab_rows(g, dir, views);
+    if (rows < PAY_ROWS) return false;
     const int pairs = (int)(views.size() + SLAB_W - 1) / SLAB_W;
     const int nub = ((int)d.det_u + SLAB_U - 1) / SLAB_U, nvb = ((int)d.det_v + rows - 1) / rows;
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
-    }
-    const double waves = (double)pairs * nub * nvb / (2 * sms);
+    const double waves = slab_waves(d, views.size(), rows);
     if (waves < (rows >= PAY_TALL ? PAY_TALL_WAVES : PAY_WAVES)) return false;
     const int n0 = (int)(dir == 0 ? d.vol_x : d.vol_y), n1 = (int)(dir == 0 ? d.vol_y : d.vol_x), n2 = (int)d.vol_z;
     const int samples = std::min(pairs, 6);
@@ -1320,11 +1363,11 @@ b2t_status fp_slab_project(const b2t_geom3d *g, const b2t_params3d *p, const voi
     L.nv = d.det_v;
     L.na = d.angles;
     L.accumulate = (mode == B2T_MODE_ADD) ? 1 : 0;
-    L.rows = slab_rows(d);
     fp_scale(g->kind, dir, g->vol_scale, false, p->output_scale, L.f1, L.f2, L.mul);
     std::vector<int> views;
     for (uint32_t a = 0; a < d.angles; ++a)
         if (dirs[a] == dir) views.push_back((int)a);
+    if (!views.empty()) L.rows = slab_rows(g, dir, views);
     const size_t smem = (size_t)SLAB_SLOTS * SLAB_SLOT * sizeof(float2) + SLAB_STAGES * 2 * sizeof(uint64_t) +
                         SLAB_SLOTS * sizeof(SlabInfo) + 2 * sizeof(int);
     for (size_t c0 = 0; c0 < views.size() && st == B2T_OK; c0 += SLAB_MAX_VIEWS) {

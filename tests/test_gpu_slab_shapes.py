@@ -122,3 +122,24 @@ def test_16_bit_choice_of_kernel(astra, case, dtype, monkeypatch):
     _stats(L)
     pr.fp(vol.float(), full)
     assert _stats(L)[3] == 0
+
+
+@pytest.mark.parametrize("rows", [161, 180, 230, 330, 358])
+@pytest.mark.parametrize("nz", [40, 120, 300])
+def test_row_blocks_full_and_equal(astra, orc, rows, nz, monkeypatch):
+    """Enough CTAs for full blocks of rows and a rest, where these leave more of
+    the detector beside the volume's shadow, and equal blocks; short and tall
+    volumes, a detector shifted along z."""
+    views = 1000
+    out = np.zeros((views, 12))
+    for i in range(views):
+        t = 2 * np.pi * i / views
+        u, r = np.array([np.cos(t), np.sin(t), 0.0]), np.array([np.sin(t), -np.cos(t), 0.0])
+        out[i] = np.concatenate([r * 60.0, -r * 20.0 + [0.0, 0.0, 13.0], 1.1 * u, [0.0, 0.0, 1.2]])
+    pr = astra.Projector3D(astra.create_proj_geom('cone_vec', rows, 33, out), astra.create_vol_geom(20, 18, nz))
+    v = torch.rand(pr.vol_shape, device='cuda')
+    a = pr.fp(v, torch.zeros(pr.proj_shape, device='cuda'))
+    monkeypatch.setenv("B2T_FP_PATH", "cells")
+    b = pr.fp(v, torch.zeros(pr.proj_shape, device='cuda'))
+    assert float(b.abs().max()) > 0
+    assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) < 2e-6
