@@ -721,15 +721,27 @@ FPCells::FPCells() = default;
 FPCells::~FPCells() = default;
 
 b2t_status fp3d_cells_build(const b2t_geom3d *g, const b2t_params3d *p, const void *vol, size_t vol_pitch,
-                            int32_t dtype, const bool need[3], cudaStream_t s, FPCells &c)
+                            int32_t dtype, const bool need[3], bool choose, cudaStream_t s, FPCells &c)
 {
     if (vol_pitch == 0) vol_pitch = g->dims.vol_x;
     std::vector<int> dirs(g->dims.angles);
     for (uint32_t a = 0; a < g->dims.angles; ++a) dirs[a] = dominant_axis(g->kind, g->views[a], g->dims);
-    bool slab[3] = {false, false, false};
-    for (int dir = 0; dir < 2; ++dir)
-        slab[dir] = need[dir] && (dtype == B2T_F32 || fp_slab_pays(g, dir, dirs)) && fp_slab_eligible(g, p, dir, dirs);
-    if (dtype == B2T_F32) return build_cells_t<float>(g, vol, vol_pitch, need, slab, s, c);
+    bool slab[3] = {false, false, false}, cells_chosen = false;
+    for (int dir = 0; dir < 2; ++dir) {
+        if (!need[dir]) continue;
+        if (dtype != B2T_F32) {
+            slab[dir] = fp_slab_pays(g, dir, dirs, dtype) && fp_slab_eligible(g, p, dir, dirs);
+        } else if (fp_slab_eligible(g, p, dir, dirs)) {
+            slab[dir] = !choose || fp_slab_pays(g, dir, dirs, dtype);
+            cells_chosen = cells_chosen || !slab[dir];
+        }
+    }
+    if (dtype == B2T_F32) {
+        const b2t_status st = build_cells_t<float>(g, vol, vol_pitch, need, slab, s, c);
+        if (st != B2T_ERR_NO_MEMORY || !cells_chosen) return st;
+        clear_error();  // the slab copy is half the size
+        return fp3d_cells_build(g, p, vol, vol_pitch, dtype, need, false, s, c);
+    }
     if (dtype == B2T_F16) return build_cells_t<__half>(g, vol, vol_pitch, need, slab, s, c);
     return build_cells_t<__nv_bfloat16>(g, vol, vol_pitch, need, slab, s, c);
 }
@@ -757,7 +769,7 @@ b2t_status fp3d_cells(const b2t_geom3d *g, const b2t_params3d *p, const void *vo
     bool need[3] = {false, false, false};
     for (int dd : dirs) need[dd] = true;
     FPCells c;
-    B2T_TRY(fp3d_cells_build(g, p, vol, vol_pitch, dtype, need, s, c));
+    B2T_TRY(fp3d_cells_build(g, p, vol, vol_pitch, dtype, need, true, s, c));
     if (dtype == B2T_F32) return project_cells_t<float>(g, p, c, proj, proj_pitch, mode, dirs, s);
     if (dtype == B2T_F16) return project_cells_t<__half>(g, p, c, proj, proj_pitch, mode, dirs, s);
     return project_cells_t<__nv_bfloat16>(g, p, c, proj, proj_pitch, mode, dirs, s);

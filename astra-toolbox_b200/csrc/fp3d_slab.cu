@@ -1214,44 +1214,55 @@ bool fp_slab_eligible(const b2t_geom3d *g, const b2t_params3d *p, int dir, const
 //  - PAY_ROWS a CTA: a 256^3 volume x 360 views on 32 detector rows (11 waves) 1.78, 64
 //    rows 1.10, 96 (two blocks of them) 0.86 to 0.95, 128 to 160 0.69 to 0.87;
 //  - PAY_FIT, the share of slice boxes that fit a buffer (neighbouring views far
-//    apart, magnified or coarse detectors): 0.65 (spacing 1.6 texels) 1.38, 0.83 (320^3 x
-//    90) 0.89, 0.87 (256^3, magnified five times) 0.96, 320^3 x 45 1.11, above that as
-//    the rows say;
+//    apart, magnified or coarse detectors): 0.65 (spacing 1.6 texels) 1.38, 0.75 (256^3 x
+//    90, pixels of a texel) 1.08, above that as the rows say; PAY_IN_FIT in launches of
+//    PAY_IN_WAVES whose boxes lie inside (PAY_IN): 256^3 x 64 (fit 0.79, use 0.92) and
+//    320^3 x 64 (0.61, 0.91) 0.89, but 256^3 x 45 (0.64, 4 waves) 1.04 and 320^3 x 45
+//    (0.51) 1.10;
 //  - PAY_USE, the share of a box inside the volume: a source three quarters of a
-//    128^3 volume's width away 0.74 1.08, 256^3 and 0.6 pixels 0.8 0.73.
+//    128^3 volume's width away 0.74 1.08, 256^3 and 0.6 pixels 0.8 0.73; of few waves
+//    PAY_TALL_USE (150^3 x 100, magnified six times, 3.4 waves 0.77 1.18).
 // The shares are those of a sample: up to six pairs of neighbouring views (less
 // the worst, a pair on either side of the other direction's views), three
 // columns of tiles, the first and the middle row of them, five slices.  About 7 us
 // of host time, asked only of launches of PAY_TALL_WAVES, several hundred us.
-constexpr double PAY_WAVES = 3.5, PAY_FIT = 0.9, PAY_USE = 0.75, PAY_TALL_WAVES = 2.2, PAY_TALL_FIT = 0.99;
+//
+// FP32 data: the slab unless a launch of PAY_F32_WAVES or more has boxes that miss
+// both the buffers and the volume, where slices in global memory cost it more than
+// the cells' twice as large copy: fits below PAY_F32_LOOSE of a use below
+// PAY_F32_USE, PAY_F32_FIT below PAY_IN, PAY_F32_IN above it.  Slab and cells, cone,
+// 1.5 times magnified, fit and use: 256^3 x 360 views, pixels of 1.5 0.95 0.82, 5.88 and
+// 6.18 ms; 1.8 0.86 0.76, 5.00 and 4.72; 2.1 0.56 0.76, 4.67 and 3.72; 4.5 0 0.75, 2.44 and
+// 1.33; 256^3 x 90, 1.5 0.75 0.79, 2.01 and 1.91; 256^3 x 128 0.85 0.82, 2.49 and 2.53; pixels of
+// 1.2, 256^3 x 64 0.79 0.92, 1.64 and 1.86; 320^3 x 64 0.61 0.91, 3.13 and 3.75; 320^3 x 32
+// 0.32 0.91, 2.21 and 2.44.  A pair in the middle of half the views is looked at first,
+// and where all its boxes fit, as they mostly do, nothing else (0.5 us a direction;
+// the whole sample 2 to 3 us, which smaller launches, of 130 us, would feel).
+constexpr double PAY_WAVES = 3.5, PAY_FIT = 0.9, PAY_USE = 0.75, PAY_TALL_WAVES = 2.2, PAY_TALL_FIT = 0.99, PAY_TALL_USE = 0.85;
+constexpr double PAY_IN = 0.88, PAY_IN_WAVES = 5.0, PAY_IN_FIT = 0.6;
+constexpr double PAY_F32_WAVES = 0.5, PAY_F32_LOOSE = 0.87, PAY_F32_USE = 0.78, PAY_F32_FIT = 0.77, PAY_F32_IN = 0.3;
 constexpr int PAY_ROWS = 96, PAY_TALL = 128;
 
-bool fp_slab_pays(const b2t_geom3d *g, int dir, const std::vector<int> &dirs)
+struct SlabShares {
+    double fit, use;
+};
+SlabShares slab_shares(const b2t_geom3d *g, int dir, const std::vector<uint32_t> &views, int rows, int samples, int tiles)
 {
-    if (slab_path('s')) return true;
     const b2t_dims3d &d = g->dims;
-    std::vector<uint32_t> views;
-    for (uint32_t a = 0; a < d.angles; ++a)
-        if (dirs[a] == dir) views.push_back(a);
-    if (views.empty()) return true;
-    const int rows = slab_rows(g, dir, views);
-    if (rows < PAY_ROWS) return false;
     const int pairs = (int)(views.size() + SLAB_W - 1) / SLAB_W;
     const int nub = ((int)d.det_u + SLAB_U - 1) / SLAB_U, nvb = ((int)d.det_v + rows - 1) / rows;
-    const double waves = slab_waves(d, views.size(), rows);
-    if (waves < (rows >= PAY_TALL ? PAY_TALL_WAVES : PAY_WAVES)) return false;
     const int n0 = (int)(dir == 0 ? d.vol_x : d.vol_y), n1 = (int)(dir == 0 ? d.vol_y : d.vol_x), n2 = (int)d.vol_z;
-    const int samples = std::min(pairs, 6);
     double worst = 1.0, fit = 0.0, use = 0.0;
     for (int k = 0; k < samples; ++k) {
-        const int first = SLAB_W * (int)((2LL * k + 1) * pairs / (2 * samples));
+        // (one: not where the other direction's views part these)
+        const int first = SLAB_W * (int)((2LL * k + 1) * pairs / std::max(4, 2 * samples));
         FPView w[SLAB_W];
         for (int i = 0; i < SLAB_W; ++i)
             fp_view_coeffs(g->kind, g->views[views[std::min(first + i, (int)views.size() - 1)]], d, dir, w[i]);
         int met = 0, fits = 0;
         double inside = 0.0;
-        for (int t = 0; t < 6; ++t) {
-            const int u0 = SLAB_U * (nub * (t / 2 + 1) / 4), v0 = rows * (t % 2 ? nvb / 2 : 0);
+        for (int t = 0; t < tiles; ++t) {
+            const int u0 = SLAB_U * (nub * ((t / 2 + 1) % 3 + 1) / 4), v0 = rows * (t % 2 ? nvb / 2 : 0);
             double A1[SLAB_NC], B1[SLAB_NC], A2[SLAB_NC], B2[SLAB_NC];
             for (int c = 0; c < SLAB_NC; ++c) {
                 const FPView &V = w[c >> 2];
@@ -1296,7 +1307,31 @@ bool fp_slab_pays(const b2t_geom3d *g, int dir, const std::vector<int> &dirs)
         use += inside / met;
     }
     if (samples > 1) fit = (fit - worst) / (samples - 1);
-    return fit >= (waves < PAY_WAVES ? PAY_TALL_FIT : PAY_FIT) && use / samples >= PAY_USE;
+    return {fit, use / samples};
+}
+
+bool fp_slab_pays(const b2t_geom3d *g, int dir, const std::vector<int> &dirs, int32_t dtype)
+{
+    if (slab_path('s')) return true;
+    const b2t_dims3d &d = g->dims;
+    std::vector<uint32_t> views;
+    for (uint32_t a = 0; a < d.angles; ++a)
+        if (dirs[a] == dir) views.push_back(a);
+    if (views.empty()) return true;
+    const int rows = slab_rows(g, dir, views);
+    const bool f32 = dtype == B2T_F32;
+    if (!f32 && rows < PAY_ROWS) return false;
+    const int pairs = (int)(views.size() + SLAB_W - 1) / SLAB_W;
+    const double waves = slab_waves(d, views.size(), rows);
+    if (f32) {
+        if (waves < PAY_F32_WAVES || slab_shares(g, dir, views, rows, 1, 2).fit == 1.0) return true;
+        const SlabShares s = slab_shares(g, dir, views, rows, std::min(pairs, 6), 2);
+        return s.fit >= (s.use >= PAY_IN ? PAY_F32_IN : s.use >= PAY_F32_USE ? PAY_F32_FIT : PAY_F32_LOOSE);
+    }
+    if (waves < (rows >= PAY_TALL ? PAY_TALL_WAVES : PAY_WAVES)) return false;
+    const SlabShares s = slab_shares(g, dir, views, rows, std::min(pairs, 6), 6);
+    if (waves >= PAY_IN_WAVES && s.use >= PAY_IN) return s.fit >= PAY_IN_FIT;
+    return s.fit >= (waves < PAY_WAVES ? PAY_TALL_FIT : PAY_FIT) && s.use >= (waves < PAY_WAVES ? PAY_TALL_USE : PAY_USE);
 }
 
 size_t fp_slab_copy_bytes(const b2t_dims3d &d, int dir)

@@ -149,16 +149,19 @@ struct FPCells {
     uint32_t vol_x = 0, vol_y = 0, vol_z = 0;
 };
 // Builds the cells (or slab copies) of the marching axes marked in need[]
-// (x, y, z) for the views of g projected with parameters p.
+// (x, y, z) for the views of g projected with parameters p.  choose: FP32 data
+// may be laid out as cells where these are faster for all views of g in one
+// projection (fp_slab_pays); else slab copies wherever the views allow them, half
+// the size.
 b2t_status fp3d_cells_build(const b2t_geom3d *g, const b2t_params3d *p, const void *vol, size_t vol_pitch,
-                            int32_t dtype, const bool need[3], cudaStream_t s, FPCells &c);
+                            int32_t dtype, const bool need[3], bool choose, cudaStream_t s, FPCells &c);
 
 // TMA-staged slab forward projector (fp3d_slab.cu) for x- and y-major views
 // whose rays share the in-plane position along a detector column, any storage
 // type, no detector supersampling.
 bool fp_slab_eligible(const b2t_geom3d *g, const b2t_params3d *p, int dir, const std::vector<int> &dirs);
-// Whether it is faster than the cell kernels for 16-bit data (for FP32 it always is).
-bool fp_slab_pays(const b2t_geom3d *g, int dir, const std::vector<int> &dirs);
+// Whether it is faster than the cell kernels for data of this type.
+bool fp_slab_pays(const b2t_geom3d *g, int dir, const std::vector<int> &dirs, int32_t dtype);
 size_t fp_slab_copy_bytes(const b2t_dims3d &d, int dir);
 b2t_status fp_slab_build(const b2t_dims3d &d, const void *vol, size_t vol_pitch, int32_t dtype, int dir, void *copy,
                          cudaStream_t s);

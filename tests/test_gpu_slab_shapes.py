@@ -122,6 +122,45 @@ def test_16_bit_choice_of_kernel(astra, case, dtype, monkeypatch):
     _stats(L)
     pr.fp(vol.float(), full)
     assert _stats(L)[3] == 0
+    assert rel_l2(out["slab"].float().cpu().numpy(), full.cpu().numpy()) < tol
+
+
+# (volume, views, detector columns, rows, pixel, slab): pixels of 0.8 voxels at the
+# volume's middle and of twice their size, few views of them, and views far apart
+# that see past the volume and that do not
+@pytest.mark.parametrize("vol,views,nu,nv,px,slab", [
+    ((150, 150, 150), 200, 200, 180, 1.2, True),
+    ((150, 150, 150), 200, 110, 100, 3.0, False),
+    ((200, 200, 200), 24, 200, 200, 1.8, False),
+    ((200, 200, 200), 32, 250, 250, 1.2, True),
+    ((150, 150, 150), 16, 110, 100, 3.0, True),
+])
+def test_fp32_choice_of_kernel(astra, orc, vol, views, nu, nv, px, slab, monkeypatch):
+    """FP32 scans whose slices do not fit the slab's buffers take the cells, with
+    the slab's values; a failed allocation of theirs takes the slab."""
+    L = importlib.import_module("astra-toolbox_b200._lib")
+    nx, ny, nz = vol
+    ang = np.linspace(0, 2 * np.pi, views, endpoint=False).astype(np.float32)
+    pr = astra.Projector3D(astra.create_proj_geom('cone', px, px, nv, nu, ang, 2.0 * nx, 1.0 * nx),
+                           astra.create_vol_geom(ny, nx, nz))
+    v = torch.rand(pr.vol_shape, device='cuda', generator=torch.Generator('cuda').manual_seed(2))
+    _stats(L)
+    a = pr.fp(v, torch.zeros(pr.proj_shape, device='cuda'))
+    s = _stats(L)
+    assert (s[2] > 0, s[3] > 0) == (slab, not slab)
+    monkeypatch.setenv("B2T_FP_PATH", "slab")
+    b = pr.fp(v, torch.zeros(pr.proj_shape, device='cuda'))
+    monkeypatch.delenv("B2T_FP_PATH")
+    assert _stats(L)[3] == 0
+    # both round positions and sums in FP32
+    assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) < 2e-6
+    if not slab:
+        L.load().b2t_debug_fail_alloc(1, None)
+        try:
+            c = pr.fp(v, torch.zeros(pr.proj_shape, device='cuda'))
+        finally:
+            L.load().b2t_debug_fail_alloc(0, None)
+        assert _stats(L)[3] == 0 and torch.equal(b, c)
 
 
 @pytest.mark.parametrize("rows", [161, 180, 230, 330, 358])
