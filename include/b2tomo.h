@@ -85,8 +85,8 @@ b2t_status b2t_bp_packed_columns(uint64_t *columns);
  * kernel read from shared memory, stats[1] slices they read from the slab
  * copy in global memory (a box too large for a slice buffer), stats[2] slab
  * kernel launches, stats[3] cell kernel launches (views the slab kernel does
- * not take).  Synchronises the device.  A performance diagnostic; the
- * reference has no counterpart. */
+ * not take, or is slower for).  Synchronises the device.  A performance
+ * diagnostic; the reference has no counterpart. */
 b2t_status b2t_fp_path_stats(uint64_t stats[4]);
 /* Read and clear the path statistics of the matched (exact-transpose)
  * backprojection since the last call: stats[0] slices whose accumulation box
